@@ -264,12 +264,12 @@ __global__ void __launch_bounds__(kB2X *kB2Y) back2_kernel(Back2Args A, int G) {
     const int per = (A.nv + G - 1) / G;
     const int va = min(A.nv, g * per), vb = min(A.nv, va + per);
     const bool active = ix < A.nx && iy0 < A.ny;
+    // rows past the image repeat its last one: their taps stay inside the tile's segments
     const float x = ix < A.nx ? A.xds[ix] : 0.f;
     float y[kB2P], acc[kB2P];
 #pragma unroll
     for (int k = 0; k < kB2P; k++) {
-        const int iy = iy0 + k * kB2Y;
-        y[k] = iy < A.ny ? A.yds[iy] : 0.f;
+        y[k] = A.yds[min(iy0 + k * kB2Y, A.ny - 1)];
         acc[k] = 0.f;
     }
     const float *__restrict__ sino = A.sino + (long long)sl * A.nb * A.na;
