@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "sgb_common.cuh"
-#include "sgb_fdk_tma.cuh"
+#include "sgb_fdk_mirror.cuh"
 #include "sgb_host.h"
 #include "sgb_kernels.cuh"
 
@@ -99,6 +99,8 @@ struct sgb_plan {
     bool tma = false;
     FdkTmaArgs targs{};
     CUtensorMap tmap;
+    bool mirror = false;  // the scan's symmetry serves several voxels per geometry (sgb_fdk_mirror.cuh)
+    FdkMirrorArgs margs{};
     DevBuf flags;  // int[4]: box extents (pre-pass), error flags
     // optional stage timing
     bool timing = false;
@@ -306,6 +308,22 @@ int fdk_tma_autotune(sgb_plan *P, cudaStream_t st, bool tune) {
     return SGB_OK;
 }
 
+// The mirrored back-projector, where the scan has a symmetry and its boxes fit.
+int plan_fdk_mirror(sgb_plan *P, const sgb_image_geom *ig, cudaStream_t st) {
+    FdkMirrorArgs &M = P->margs;
+    fdk_mirror_slots(M, P->targs, P->cg.orbit, P->cg.orbit_start, ig->offsets, P->cg.offset_t);
+    if (M.nvs * (M.zm ? 2 : 1) == 1) return SGB_OK;
+    FdkTmaArgs T = P->targs;  // geometries whose pair boxes are too large keep to plain FP32 boxes
+    T.zu = 16;
+    SGB_TRY(fdk_tma_prepare(T, P->flags.as<int>(), st));
+    if (fdk_tma_choose(T)) SGB_TRY(fdk_mirror_prepare(M, P->flags.as<int>(), st, &P->mirror));
+    SGB_CUDA(cudaMemsetAsync(P->flags.p, 0, 4 * sizeof(int), st));
+    if (!P->mirror) return SGB_OK;
+    M.A.passes = 1;
+    P->tma = true;
+    return fdk_tma_encode(M.A, P->filt_buf.p, P->pitch, &P->tmap);
+}
+
 // Filtered-projection layout and back-projector choice for an FDK plan: rows padded to
 // a multiple of 8 samples (16-byte TMA strides for every storage type); the TMA-staged
 // kernel when its box fits (exhaustive pre-pass), the direct kernel otherwise.  FP32 storage
@@ -364,7 +382,10 @@ int plan_fdk_back(sgb_plan *P, const sgb_image_geom *ig, cudaStream_t st, bool t
     double ry = std::fabs(ig->deltas[1]) * (ig->dims[1] / 2.0 + std::fabs(ig->offsets[1]) + 1);
     P->tma = false;
     if (std::sqrt(rx * rx + ry * ry) < 0.9 * (g.dsd - g.dod)) {
-        SGB_TRY(fdk_tma_autotune(P, st, tune));
+        if (tune && !A.quad) SGB_TRY(plan_fdk_mirror(P, ig, st));
+        if (!P->mirror) SGB_TRY(fdk_tma_autotune(P, st, tune));
+        // quads keep the t grid that the unmirrored form's z-run anchors
+        if (tune && P->tma && A.quad) SGB_TRY(plan_fdk_mirror(P, ig, st));
         if (!P->tma && A.elem_bytes == 8) {  // pair or quad boxes too large: plain FP32 boxes
             A.elem_bytes = 4;
             A.quad = 0;
@@ -542,18 +563,19 @@ int sgb_plan_set_view_passes(sgb_plan *P, int passes) {
     SGB_REQUIRE(P && P->ct, "plan_set_view_passes: needs an FDK plan");
     SGB_REQUIRE(passes >= 1 && passes <= 8, "plan_set_view_passes: passes must be in [1, 8], got %d", passes);
     SGB_REQUIRE(passes <= P->cg.na, "plan_set_view_passes: more passes than views");
-    P->targs.passes = passes;
+    P->targs.passes = P->margs.A.passes = passes;
     return SGB_OK;
 }
 
 int sgb_plan_info(const sgb_plan *P, int *info, int n) {
     SGB_REQUIRE(P && info && n >= 5, "plan_info: bad argument");
     info[0] = P->tma ? 1 : 0;
-    info[1] = P->targs.W;
-    info[2] = P->targs.H;
+    const FdkTmaArgs &A = P->mirror ? P->margs.A : P->targs;
+    info[1] = A.W;
+    info[2] = A.H;
     info[3] = P->pitch;
-    info[4] = P->targs.zu;
-    if (n >= 6) info[5] = P->targs.passes;
+    info[4] = P->mirror ? P->margs.kz * (P->margs.zm ? 2 : 1) : A.zu;
+    if (n >= 6) info[5] = A.passes;
     if (n >= 7) info[6] = P->ct ? P->targs.elem_bytes : 4;
     if (n >= 8) info[7] = P->ct ? P->targs.quad : 0;
     return SGB_OK;
@@ -637,10 +659,17 @@ int sgb_fdk(sgb_plan *P, const float *proj, float *image, int flags, void *strea
     }
     // step 3: cbct_back (fdk.jl:78)
     if (P->tma) {
-        FdkTmaArgs T = P->targs;
-        T.image = img_dev;
-        T.mask = P->mask_dev;
-        SGB_TRY(launch_fdk_tma(T, P->tmap, st));
+        if (P->mirror) {
+            FdkMirrorArgs M = P->margs;
+            M.A.image = img_dev;
+            M.A.mask = P->mask_dev;
+            SGB_TRY(launch_fdk_mirror(M, P->tmap, st));
+        } else {
+            FdkTmaArgs T = P->targs;
+            T.image = img_dev;
+            T.mask = P->mask_dev;
+            SGB_TRY(launch_fdk_tma(T, P->tmap, st));
+        }
         P->mark(2, st);
         if (!(flags & SGB_DEVICE_PTRS))
             SGB_CUDA(cudaMemcpyAsync(image, img_dev, nvox * sizeof(float), cudaMemcpyDeviceToHost, st));

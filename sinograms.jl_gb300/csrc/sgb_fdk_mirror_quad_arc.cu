@@ -1,0 +1,12 @@
+// sgb_fdk_mirror_quad_arc.cu -- mirrored FDK back-projection of FP16 quads (F16 form), arc detector.
+#include "sgb_fdk_mirror_kernel.cuh"
+
+namespace sgb {
+
+int launch_fdk_mirror_quad_arc(const FdkMirrorArgs &M, const CUtensorMap &map, cudaStream_t st) {
+    using namespace fdkdev;
+    if (M.nvs == 4) return M.kz == 16 ? launch_mirror_k<Quad16, true, 4, false, 16>(M, map, st) : launch_mirror_k<Quad16, true, 4, false, 8>(M, map, st);
+    return M.kz == 32 ? launch_mirror_k<Quad16, true, 2, false, 32>(M, map, st) : launch_mirror_k<Quad16, true, 2, false, 16>(M, map, st);
+}
+
+}  // namespace sgb
