@@ -74,6 +74,7 @@ struct sgb_plan {
     sgb_ct_geom cg{};
     sgb_sino_geom sg{};
     int nx = 0, ny = 0, nz = 1;
+    double deltas[3] = {0, 0, 0}, offsets[3] = {0, 0, 0};
     int storage = SGB_STORE_F32;
     int npad = 0;
     std::vector<double> Hk;
@@ -91,6 +92,7 @@ struct sgb_plan {
     float scale = 1.f;
     // staging for host-pointer calls
     DevBuf in_buf, filt_buf, img_buf;
+    DevBuf inter;  // 2D stacks: the filtered slices interleaved in fours
     // F16 form: the filter's FP32 rows before they become FP16 quads, and the device words
     // (max |y| as bits, inverse scale) of the quads' power-of-two scale
     DevBuf qtmp, qword;
@@ -175,6 +177,10 @@ int plan_image(sgb_plan *P, const sgb_image_geom *ig, double ds, int ndim, cudaS
     P->ny = ig->dims[1];
     P->nz = ndim == 3 ? ig->dims[2] : 1;
     SGB_REQUIRE(P->nx > 0 && P->ny > 0 && P->nz > 0, "image dims must be positive");
+    for (int i = 0; i < ndim; i++) {
+        P->deltas[i] = ig->deltas[i];
+        P->offsets[i] = ig->offsets[i];
+    }
     std::vector<double> x = image_axis(P->nx, ig->deltas[0], ig->offsets[0], ds);
     std::vector<double> y = image_axis(P->ny, ig->deltas[1], ig->offsets[1], ds);
     SGB_TRY(upload_f32(x.data(), x.size(), 1.0, P->xds, st));
@@ -716,6 +722,43 @@ int sgb_fdk(sgb_plan *P, const float *proj, float *image, int flags, void *strea
     return plan_done(P, flags, st);
 }
 
+// Back-projection of a 2D plan's filtered slices.
+static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices, cudaStream_t st) {
+    const sgb_sino_geom &g = P->sg;
+    Back2Args A{};
+    A.mask = P->mask_dev;
+    A.trig = P->trig.as<float2>();
+    A.xds = P->xds.as<float>();
+    A.yds = P->yds.as<float>();
+    A.nb = g.nb;
+    A.na = g.na;
+    A.nx = P->nx;
+    A.ny = P->ny;
+    A.nv = g.na;
+    A.ia_skip = 1;
+    A.wb = (float)((g.nb + 1) / 2.0 + g.offset);
+    A.mode = g.kind;
+    A.dsd_ds = (float)(g.dsd / g.d);
+    A.dso_ds = (float)((g.dsd - g.dod) / g.d);
+    A.so_ds = (float)(g.source_offset / g.d);
+    A.ns = 1;
+    A.hx = A.nx;
+    A.hy = A.ny;
+    back2_window(A, P->deltas[0] / g.d, P->deltas[1] / g.d);
+    back2_slots(A, g.orbit, g.orbit_start, P->deltas, P->offsets);
+    A.sino = sino;
+    A.image = image;
+    A.nslices = nslices;
+    back2_choose(A);
+    if (A.sl == 4) {
+        const long long n = (long long)g.nb * g.na;
+        SGB_TRY(P->inter.reserve(sizeof(float) * 4 * n * floor_div_up(nslices, 4)));
+        SGB_TRY(launch_interleave4(sino, P->inter.as<float>(), n, nslices, st));
+        A.sino4 = P->inter.as<float>();
+    }
+    return launch_back2(A, st);
+}
+
 int sgb_fbp(sgb_plan *P, const float *sino, float *image, int nslices, int flags, void *stream) {
     SGB_REQUIRE(P && sino && image, "fbp: null argument");
     SGB_REQUIRE(!P->ct, "fbp: plan is a CT plan; use fdk");
@@ -735,26 +778,7 @@ int sgb_fbp(sgb_plan *P, const float *sino, float *image, int nslices, int flags
         SGB_TRY(P->img_buf.reserve(npix * sizeof(float)));
         img_dev = P->img_buf.as<float>();
     }
-    Back2Args A{};
-    A.sino = P->filt_buf.as<float>();
-    A.image = img_dev;
-    A.mask = P->mask_dev;
-    A.trig = P->trig.as<float2>();
-    A.xds = P->xds.as<float>();
-    A.yds = P->yds.as<float>();
-    A.nb = g.nb;
-    A.na = g.na;
-    A.nx = P->nx;
-    A.ny = P->ny;
-    A.nv = g.na;
-    A.ia_skip = 1;
-    A.nslices = nslices;
-    A.wb = (float)((g.nb + 1) / 2.0 + g.offset);
-    A.mode = g.kind;
-    A.dsd_ds = (float)(g.dsd / g.d);
-    A.dso_ds = (float)((g.dsd - g.dod) / g.d);
-    A.so_ds = (float)(g.source_offset / g.d);
-    SGB_TRY(launch_back2(A, st));
+    SGB_TRY(plan_back2(P, P->filt_buf.as<float>(), img_dev, nslices, st));
     P->mark(2, st);
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(image, img_dev, npix * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -794,26 +818,7 @@ int sgb_fbp_backproject(sgb_plan *P, const float *filtered, float *image, int ns
         SGB_TRY(P->img_buf.reserve(npix * sizeof(float)));
         img_dev = P->img_buf.as<float>();
     }
-    Back2Args A{};
-    A.sino = static_cast<const float *>(in_dev);
-    A.image = img_dev;
-    A.mask = P->mask_dev;
-    A.trig = P->trig.as<float2>();
-    A.xds = P->xds.as<float>();
-    A.yds = P->yds.as<float>();
-    A.nb = g.nb;
-    A.na = g.na;
-    A.nx = P->nx;
-    A.ny = P->ny;
-    A.nv = g.na;
-    A.ia_skip = 1;
-    A.nslices = nslices;
-    A.wb = (float)((g.nb + 1) / 2.0 + g.offset);
-    A.mode = g.kind;
-    A.dsd_ds = (float)(g.dsd / g.d);
-    A.dso_ds = (float)((g.dsd - g.dod) / g.d);
-    A.so_ds = (float)(g.source_offset / g.d);
-    SGB_TRY(launch_back2(A, st));
+    SGB_TRY(plan_back2(P, static_cast<const float *>(in_dev), img_dev, nslices, st));
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(image, img_dev, npix * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (flags & SGB_ASYNC) return SGB_OK;
@@ -960,6 +965,12 @@ static int back2_seam(float *image, const float *sino, int nb, int na, const dou
     A.dsd_ds = (float)(dsd / ds);
     A.dso_ds = (float)(dso / ds);
     A.so_ds = (float)(source_offset / ds);
+    A.ns = 1;
+    A.hx = nx;
+    A.hy = ny;
+    // the axes are the caller's, spaced as they like: their mean spacing
+    back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0);
+    back2_choose(A);
     SGB_TRY(launch_back2(A, st));
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(image, img_dev, sizeof(float) * (size_t)nx * ny, cudaMemcpyDeviceToHost, st));

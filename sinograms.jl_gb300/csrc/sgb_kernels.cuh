@@ -92,6 +92,7 @@ int launch_fdk_back(const FdkArgs &A, cudaStream_t st);
 // ---------------------------------------------- 2D pixel-driven back-projection
 struct Back2Args {
     const float *sino;     // (nb, na, nslices)
+    const float *sino4;    // stacks: four slices at a time interleaved, (4, nb, na, ceil(nslices / 4)), or null
     float *image;          // (nx, ny, nslices)
     const uint8_t *mask;   // (nx, ny) or null
     const float2 *trig;    // nv used views: (sin, cos)
@@ -100,8 +101,44 @@ struct Back2Args {
     float wb;
     int mode;              // SGB_PAR, SGB_ARC, SGB_FLAT
     float dsd_ds, dso_ds, so_ds;
+    // Symmetry (sgb_back2_kernel.cuh): the first hx x hy pixels, each with its images in ns slots.  Slot j
+    // takes view (sgn v + off) mod the period, its bins reversed if rev; map: 1 flips x, 2 flips y, 4
+    // swaps them first.
+    struct Slot {
+        int map, sgn, off, rev;
+    };
+    int sl, split;  // slices per CTA (1 or 4) and CTAs that share a tile's views (back2_choose)
+    int w, vc;  // staged bins per segment (<= 256; longer ones read global memory) and views per chunk
+    int ns, hx, hy, turn, half;
+    Slot slot[4];
 };
+constexpr int kB2X = 32, kB2Y = 8;  // pixels of a 2D tile that its 256 threads take at a time
+// such passes: rows of a tile / 8.  Two where a pixel has 16 sums, which leaves registers for a third
+// CTA per SM
+template <int NS, int SL>
+constexpr int kB2P = NS * SL > 4 ? 2 : 4;
+// CTAs that share an SM, by their registers and staged segments
+template <int NS, int SL>
+constexpr int kB2Ctas = NS * SL == 1 ? 5 : 3;
+constexpr int kB2V = 32;   // views per chunk, at most
+constexpr int kB2W = 256;  // staged bins per view and slot, at most; the last two stay zero
+// bytes of staged segments, two buffers: kB2Ctas CTAs per SM
+template <int NS, int SL>
+constexpr int kB2Seg = (NS * SL == 1 ? 40 : 64) * 1024;
+// w and, for a plan's geometry, the slots (ns = 1, hx = nx, hy = ny before)
+void back2_window(Back2Args &A, double dx, double dy);
+void back2_slots(Back2Args &A, double orbit, double orbit_start, const double *deltas, const double *offsets);
+// The launch predicted to be the fastest: with or without the slots, slices one by one or in fours, and
+// the view split.
+void back2_choose(Back2Args &A);
 int launch_back2(const Back2Args &A, cudaStream_t st);
+// (n, nslices) -> (4, n, ceil(nslices / 4)); the last group's missing slices are zeros
+int launch_interleave4(const float *in, float *out, long long n, int nslices, cudaStream_t st);
+int launch_back2_par(const Back2Args &A, cudaStream_t st);
+int launch_back2_flat(const Back2Args &A, cudaStream_t st);
+int launch_back2_arc(const Back2Args &A, cudaStream_t st);
+int launch_back2_arc_narrow(const Back2Args &A, cudaStream_t st);
+int launch_back2_arc_exact(const Back2Args &A, cudaStream_t st);
 
 // ------------------------------------------------------- distance-driven pair
 struct BddArgs {
