@@ -741,11 +741,9 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
     A.dsd_ds = (float)(g.dsd / g.d);
     A.dso_ds = (float)((g.dsd - g.dod) / g.d);
     A.so_ds = (float)(g.source_offset / g.d);
-    A.ns = 1;
-    A.hx = A.nx;
-    A.hy = A.ny;
     back2_window(A, P->deltas[0] / g.d, P->deltas[1] / g.d);
-    back2_slots(A, g.orbit, g.orbit_start, P->deltas, P->offsets);
+    A.sym = scan_slots(g.kind, g.na, P->nx, P->ny, 2.0 * A.wb == g.nb + 1.0, g.source_offset == 0, g.orbit, g.orbit_start,
+                       P->deltas, P->offsets, true);
     A.sino = sino;
     A.image = image;
     A.nslices = nslices;
@@ -965,9 +963,7 @@ static int back2_seam(float *image, const float *sino, int nb, int na, const dou
     A.dsd_ds = (float)(dsd / ds);
     A.dso_ds = (float)(dso / ds);
     A.so_ds = (float)(source_offset / ds);
-    A.ns = 1;
-    A.hx = nx;
-    A.hy = ny;
+    A.sym = ScanSlots{1, nx, ny, 0, 0, {{0, 1, 0, 0}}};
     // the axes are the caller's, spaced as they like: their mean spacing
     back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0);
     back2_choose(A);

@@ -172,15 +172,20 @@ void back2_window(Back2Args &A, double dx, double dy) {
     A.w = span < 256 ? ((int)span + 7) / 8 * 8 : 256;
 }
 
-// Slots of a 2D scan on a uniform image grid (sgb_back2_kernel.cuh): which pixels and views share
-// geometry.  Needs the grid centred (offsets 0) on the axes that a slot mirrors, and for slots whose bins
-// run the other way a centred detector.
-void back2_slots(Back2Args &A, double orbit, double orbit_start, const double *deltas, const double *offsets) {
-    const double step = orbit / A.na, turns = std::fabs(orbit) / 360.0;
-    const bool whole = turns >= 1 && turns == std::floor(turns);
-    A.half = A.mode == SGB_PAR && std::fabs(orbit) == 180.0;  // views 180 degrees apart are each other reversed
-    if (!(whole || A.half) || A.ia_skip != 1) return;
-    const int period = A.half ? 2 * A.na : A.na;
+// Which pixels and views share geometry: needs the grid centred (offsets 0) on the axes that a slot
+// mirrors, and for slots whose bins run the other way a centred detector.
+ScanSlots scan_slots(int kind, int na, int nx, int ny, bool centred, bool source_centred, double orbit,
+                     double orbit_start, const double *deltas, const double *offsets, bool prefer_turn) {
+    ScanSlots S{};
+    S.ns = 1;
+    S.hx = nx;
+    S.hy = ny;
+    S.slot[0].sgn = 1;
+    const double step = orbit / na, turns = std::fabs(orbit) / 360.0;
+    const bool whole = turns >= 1 && turns == std::floor(turns), half = kind == SGB_PAR && std::fabs(orbit) == 180.0;
+    if (!(whole || half)) return S;
+    S.half = half;
+    const int period = half ? 2 * na : na;
     auto views = [&](double angle, int *off) {  // `angle` as a whole number of views
         const double q = angle / step, r = std::nearbyint(q);
         if (!(std::fabs(q - r) < 1e-9 * std::max(1.0, std::fabs(q)))) return false;
@@ -188,42 +193,41 @@ void back2_slots(Back2Args &A, double orbit, double orbit_start, const double *d
         *off = (int)(m < 0 ? m + period : m);
         return true;
     };
-    const bool cx = offsets[0] == 0, cy = offsets[1] == 0, square = A.nx == A.ny && std::fabs(deltas[0]) == std::fabs(deltas[1]);
-    const bool centred = 2.0 * A.wb == A.nb + 1.0;
-    int o90, o180, ox, oy;
-    const bool turn90 = cx && cy && square && views(90, &o90) && (centred || !A.half);
-    const bool turn180 = cx && cy && views(180, &o180) && (centred || !A.half);
-    const bool mirror = centred && A.so_ds == 0;
+    const bool cx = offsets[0] == 0, cy = offsets[1] == 0, square = nx == ny && std::fabs(deltas[0]) == std::fabs(deltas[1]);
+    int o90 = 0, o180 = 0, ox = 0, oy = 0;
+    const bool turn90 = cx && cy && square && views(90, &o90) && (centred || !half);
+    const bool turn180 = cx && cy && views(180, &o180) && (centred || !half);
+    const bool mirror = centred && source_centred;
     const bool mx = mirror && cx && views(-2 * orbit_start, &ox), my = mirror && cy && views(180 - 2 * orbit_start, &oy);
-    auto slot = [&](int j, int map, int sgn, int off, int rev) { A.slot[j] = {map, sgn, off, rev}; };
-    slot(0, 0, 1, 0, 0);
-    if (turn90) {
-        A.ns = 4;
-        A.turn = 1;
-        A.hx = A.hy = (A.nx + 1) / 2;
+    const bool both = mx && my && turn180;
+    if (turn90 && (prefer_turn || !both)) {
+        S.ns = 4;
+        S.turn = 1;
+        S.hx = S.hy = (nx + 1) / 2;
         const bool same = (deltas[0] > 0) == (deltas[1] > 0);  // (x, y) -> (-y, x) in pixel indices
         for (int j = 1; j < 4; j++)
-            slot(j, j == 2 ? 3 : 4 + ((j == 1) == same ? 1 : 2), 1, (int)((long long)j * o90 % period), 0);
-    } else if (mx && my && turn180) {
-        A.ns = 4;
-        A.hx = (A.nx + 1) / 2;
-        A.hy = (A.ny + 1) / 2;
-        slot(1, 1, -1, ox, 1);
-        slot(2, 2, -1, oy, 1);
-        slot(3, 3, 1, o180, 0);
+            S.slot[j] = {j == 2 ? 3 : 4 + ((j == 1) == same ? 1 : 2), 1, (int)((long long)j * o90 % period), 0};
+    } else if (both) {
+        S.ns = 4;
+        S.hx = (nx + 1) / 2;
+        S.hy = (ny + 1) / 2;
+        S.slot[1] = {1, -1, ox, 1};
+        S.slot[2] = {2, -1, oy, 1};
+        S.slot[3] = {3, 1, o180, 0};
     } else if (turn180) {
-        A.ns = 2;
-        A.hy = (A.ny + 1) / 2;
-        slot(1, 3, 1, o180, 0);
+        S.ns = 2;
+        S.hy = (ny + 1) / 2;
+        S.slot[1] = {3, 1, o180, 0};
     } else if (mx) {
-        A.ns = 2;
-        A.hx = (A.nx + 1) / 2;
-        slot(1, 1, -1, ox, 1);
+        S.ns = 2;
+        S.hx = (nx + 1) / 2;
+        S.slot[1] = {1, -1, ox, 1};
     } else if (my) {
-        A.ns = 2;
-        A.hy = (A.ny + 1) / 2;
-        slot(1, 2, -1, oy, 1);
+        S.ns = 2;
+        S.hy = (ny + 1) / 2;
+        S.slot[1] = {2, -1, oy, 1};
     }
+    return S;
 }
 
 void back2_choose(Back2Args &A) {
@@ -234,10 +238,10 @@ void back2_choose(Back2Args &A) {
     const int sms = std::max(1, num_sms());
     Back2Args best = A;
     double best_us = 1e30;
-    for (int ns : {A.ns, 1}) {
+    for (int ns : {A.sym.ns, 1}) {
         for (int sl : {1, 4}) {
             if (sl == 4 && A.nslices == 1) continue;
-            const int p = ns * sl > 4 ? kB2P<4, 4> : kB2P<1, 1>, hx = ns > 1 ? A.hx : A.nx, hy = ns > 1 ? A.hy : A.ny;
+            const int p = ns * sl > 4 ? kB2P<4, 4> : kB2P<1, 1>, hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
             const long long groups = floor_div_up(A.nslices, sl);
             const long long tiles = (long long)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * p) * groups;
             const double view = 0.0015 * (p * (geometry + ns * (sl == 1 ? 4 : 10)) + 12 + ns * A.w / 48.0);
@@ -253,12 +257,12 @@ void back2_choose(Back2Args &A) {
                                   (sl == 4 ? 3 + 8e-6 * A.nb * A.na * A.nslices / 6e3 : 0);
                 if (us < best_us) {
                     best_us = us;
-                    best.ns = ns;
+                    best.sym.ns = ns;
                     best.sl = sl;
                     best.split = g;
-                    best.hx = hx;
-                    best.hy = hy;
-                    best.turn = ns > 1 ? A.turn : 0;
+                    best.sym.hx = hx;
+                    best.sym.hy = hy;
+                    best.sym.turn = ns > 1 ? A.sym.turn : 0;
                 }
             }
         }

@@ -27,7 +27,7 @@
 //   SL  slices of a stack see a pixel alike: one 16-byte load per bin for four of them;
 //   NS  so do the images of a pixel under the scan's symmetry, each in its own view ("slots"): the
 //       quarter turns of a square image where 90 degrees are a whole number of views, else reflections
-//       in x and y (whose bins run the other way: staged reversed), else a half turn (back2_slots).
+//       in x and y (whose bins run the other way: staged reversed), else a half turn (scan_slots).
 #pragma once
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -150,29 +150,6 @@ __device__ __forceinline__ void b2_tap(uint32_t a, float wa, float wb, float (&a
     }
 }
 
-// Slot j's row of the sinogram for view v, and whether its bins run the other way.
-__device__ __forceinline__ int b2_slot_view(const Back2Args &A, int j, int v, bool *rev) {
-    const int period = A.half ? 2 * A.na : A.na;
-    int u = A.slot[j].sgn * v + A.slot[j].off;  // in (-period, 2 period)
-    u = u < 0 ? u + period : (u >= period ? u - period : u);
-    *rev = (A.slot[j].rev != 0) != (u >= A.na);  // half turns: a view 180 degrees on is the view reversed
-    return u >= A.na ? u - A.na : u;
-}
-
-// Index of pixel (ix, iy)'s image in slot j; false when it belongs to another pixel or slot (pixels on
-// a mirror are their own images, those on a quarter turn's seam appear twice).
-__device__ __forceinline__ bool b2_slot_pixel(const Back2Args &A, int j, int ix, int iy, size_t *idx) {
-    if (ix >= A.hx || iy >= A.hy) return false;
-    const int f = A.slot[j].map;
-    const bool mx = 2 * ix == A.nx - 1, my = 2 * iy == A.ny - 1;
-    if (A.turn ? my && (!mx || j > 0) : (f & 1 && A.hx < A.nx && mx) || (f & 2 && A.hy < A.ny && my)) return false;
-    int px = f & 4 ? iy : ix, py = f & 4 ? ix : iy;
-    if (f & 1) px = A.nx - 1 - px;
-    if (f & 2) py = A.ny - 1 - py;
-    *idx = px + (size_t)A.nx * py;
-    return true;
-}
-
 __device__ __forceinline__ void b2_copy4(uint32_t dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -207,14 +184,14 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
 #pragma unroll
         for (int j = 0; j < NS; j++) {
             size_t idx;
-            if (b2_slot_pixel(A, j, ix, iy0 + k * kB2Y, &idx)) active |= !A.mask || A.mask[idx];
+            if (slot_pixel(A.sym, A.nx, A.ny, j, ix, iy0 + k * kB2Y, &idx)) active |= !A.mask || A.mask[idx];
         }
     // rows past the domain repeat its last one: their taps stay inside the tile's segments
-    const float x = A.xds[min(ix, A.hx - 1)];
+    const float x = A.xds[min(ix, A.sym.hx - 1)];
     float y[P], acc[P][NS][SL];
 #pragma unroll
     for (int k = 0; k < P; k++) {
-        y[k] = A.yds[min(iy0 + k * kB2Y, A.hy - 1)];
+        y[k] = A.yds[min(iy0 + k * kB2Y, A.sym.hy - 1)];
 #pragma unroll
         for (int j = 0; j < NS; j++)
 #pragma unroll
@@ -238,8 +215,8 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
         if (cn < nchunk && tid < 4 * VC) {  // lane group of 4 = one view's four corners
             const int v = tid >> 2, cr = tid & 3;
             const float2 sc = v < nvn ? A.trig[vn + v] : make_float2(0.f, 1.f);
-            const float cx = A.xds[cr & 1 ? min(A.hx, ix0 + kB2X) - 1 : ix0];
-            const float cy = A.yds[cr & 2 ? min(A.hy, iy00 + T) - 1 : iy00];
+            const float cx = A.xds[cr & 1 ? min(A.sym.hx, ix0 + kB2X) - 1 : ix0];
+            const float cy = A.yds[cr & 2 ? min(A.sym.hy, iy00 + T) - 1 : iy00];
             float a, b, w;
             bool fr, in;
             b2_col<M>(A, cx, sc.x, sc.y, &a, &b);
@@ -305,7 +282,7 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
                 const int v = i / NS, j = i % NS;
                 if (form_s[bn][v] > V_CHECKED) continue;
                 bool rev = false;
-                const int row = NS == 1 ? vn + v : b2_slot_view(A, j, vn + v, &rev);
+                const int row = NS == 1 ? vn + v : slot_view(A.sym, A.na, j, vn + v, &rev);
                 const int lo = lo_s[bn][v], len = len_s[bn][v];
                 // entry e holds bin lo + e, counted from the other end when the slot runs the other way
                 const long long o = row * vstride + (rev ? A.nb - 1 - lo : lo);
@@ -386,7 +363,7 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
 #pragma unroll
                     for (int j = 0; j < NS; j++) {
                         bool rev = false;
-                        const int row = NS == 1 ? v : b2_slot_view(A, j, v, &rev);
+                        const int row = NS == 1 ? v : slot_view(A.sym, A.na, j, v, &rev);
                         const long long o = row * vstride + (rev ? nbm1 - il1 : il1);
                         const int step = rev ? -1 : 1;
                         if constexpr (SL == 4) {
@@ -404,7 +381,7 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
     }
     auto store = [&](int k, int j, int s, float v) {
         size_t idx;
-        if (sl0 + s >= A.nslices || !b2_slot_pixel(A, j, ix, iy0 + k * kB2Y, &idx)) return;
+        if (sl0 + s >= A.nslices || !slot_pixel(A.sym, A.nx, A.ny, j, ix, iy0 + k * kB2Y, &idx)) return;
         A.image[(size_t)(sl0 + s) * A.nx * A.ny + idx] = (A.mask && !A.mask[idx]) ? 0.f : v;
     };
     if (G == 1) {
@@ -446,7 +423,7 @@ int launch_slots(Back2Args A, cudaStream_t st) {
     SGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, seg));
     A.vc = std::min(kB2V, seg / 2 / (NS * A.w * 4 * SL));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(floor_div_up(A.hx, kB2X), floor_div_up(A.hy, kB2Y * kB2P<NS, SL>), groups * G);
+    cfg.gridDim = dim3(floor_div_up(A.sym.hx, kB2X), floor_div_up(A.sym.hy, kB2Y * kB2P<NS, SL>), groups * G);
     cfg.blockDim = dim3(kB2X * kB2Y);
     cfg.dynamicSmemBytes = seg;
     cfg.stream = st;
@@ -468,8 +445,8 @@ int launch_slots(Back2Args A, cudaStream_t st) {
 template <int M>
 int launch(const Back2Args &A, cudaStream_t st) {
     if (A.sl == 4)
-        return A.ns == 4 ? launch_slots<M, 4, 4>(A, st) : (A.ns == 2 ? launch_slots<M, 2, 4>(A, st) : launch_slots<M, 1, 4>(A, st));
-    return A.ns == 4 ? launch_slots<M, 4, 1>(A, st) : (A.ns == 2 ? launch_slots<M, 2, 1>(A, st) : launch_slots<M, 1, 1>(A, st));
+        return A.sym.ns == 4 ? launch_slots<M, 4, 4>(A, st) : (A.sym.ns == 2 ? launch_slots<M, 2, 4>(A, st) : launch_slots<M, 1, 4>(A, st));
+    return A.sym.ns == 4 ? launch_slots<M, 4, 1>(A, st) : (A.sym.ns == 2 ? launch_slots<M, 2, 1>(A, st) : launch_slots<M, 1, 1>(A, st));
 }
 
 }  // namespace back2

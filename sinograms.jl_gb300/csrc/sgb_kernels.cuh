@@ -90,6 +90,44 @@ struct FdkArgs {
 int launch_fdk_back(const FdkArgs &A, cudaStream_t st);
 
 // ---------------------------------------------- 2D pixel-driven back-projection
+// Symmetry of a 2D scan on a centred image grid: a pixel and its images, each in the view that sees it
+// alike.  Slot j takes view (sgn v + off) mod the period, its bins reversed if rev; map: 1 flips x, 2
+// flips y, 4 swaps them first.  Pixels 0 <= ix < hx, 0 <= iy < hy and their images make up the image.
+struct ScanSlots {
+    struct Slot {
+        int map, sgn, off, rev;
+    };
+    int ns, hx, hy;
+    int turn;  // 1: quarter turns
+    int half;  // 1: the views cover half a turn (parallel beams); a view 180 degrees on is it reversed
+    Slot slot[4];
+};
+// centred: the detector's bins are symmetric about the central ray; prefer_turn: quarter turns before
+// reflections where the scan has both.
+ScanSlots scan_slots(int kind, int na, int nx, int ny, bool centred, bool source_centred, double orbit,
+                     double orbit_start, const double *deltas, const double *offsets, bool prefer_turn);
+// slot j's view of view v, and whether its bins run the other way
+inline __host__ __device__ int slot_view(const ScanSlots &S, int na, int j, int v, bool *rev) {
+    const int period = S.half ? 2 * na : na;
+    int u = S.slot[j].sgn * v + S.slot[j].off;  // in (-period, 2 period)
+    u = u < 0 ? u + period : (u >= period ? u - period : u);
+    *rev = (S.slot[j].rev != 0) != (u >= na);
+    return u >= na ? u - na : u;
+}
+// Index of pixel (ix, iy)'s image in slot j; false when it belongs to another pixel or slot (pixels on
+// a mirror are their own images, those on a quarter turn's seam appear twice).
+inline __host__ __device__ bool slot_pixel(const ScanSlots &S, int nx, int ny, int j, int ix, int iy, size_t *idx) {
+    if (ix >= S.hx || iy >= S.hy) return false;
+    const int f = S.slot[j].map;
+    const bool mx = 2 * ix == nx - 1, my = 2 * iy == ny - 1;
+    if (S.turn ? my && (!mx || j > 0) : (f & 1 && S.hx < nx && mx) || (f & 2 && S.hy < ny && my)) return false;
+    int px = f & 4 ? iy : ix, py = f & 4 ? ix : iy;
+    if (f & 1) px = nx - 1 - px;
+    if (f & 2) py = ny - 1 - py;
+    *idx = px + (size_t)nx * py;
+    return true;
+}
+
 struct Back2Args {
     const float *sino;     // (nb, na, nslices)
     const float *sino4;    // stacks: four slices at a time interleaved, (4, nb, na, ceil(nslices / 4)), or null
@@ -101,16 +139,9 @@ struct Back2Args {
     float wb;
     int mode;              // SGB_PAR, SGB_ARC, SGB_FLAT
     float dsd_ds, dso_ds, so_ds;
-    // Symmetry (sgb_back2_kernel.cuh): the first hx x hy pixels, each with its images in ns slots.  Slot j
-    // takes view (sgn v + off) mod the period, its bins reversed if rev; map: 1 flips x, 2 flips y, 4
-    // swaps them first.
-    struct Slot {
-        int map, sgn, off, rev;
-    };
     int sl, split;  // slices per CTA (1 or 4) and CTAs that share a tile's views (back2_choose)
     int w, vc;  // staged bins per segment (<= 256; longer ones read global memory) and views per chunk
-    int ns, hx, hy, turn, half;
-    Slot slot[4];
+    ScanSlots sym;
 };
 constexpr int kB2X = 32, kB2Y = 8;  // pixels of a 2D tile that its 256 threads take at a time
 // such passes: rows of a tile / 8.  Two where a pixel has 16 sums, which leaves registers for a third
@@ -125,9 +156,8 @@ constexpr int kB2W = 256;  // staged bins per view and slot, at most; the last t
 // bytes of staged segments, two buffers: kB2Ctas CTAs per SM
 template <int NS, int SL>
 constexpr int kB2Seg = (NS * SL == 1 ? 40 : 64) * 1024;
-// w and, for a plan's geometry, the slots (ns = 1, hx = nx, hy = ny before)
+// sets w
 void back2_window(Back2Args &A, double dx, double dy);
-void back2_slots(Back2Args &A, double orbit, double orbit_start, const double *deltas, const double *offsets);
 // The launch predicted to be the fastest: with or without the slots, slices one by one or in fours, and
 // the view split.
 void back2_choose(Back2Args &A);

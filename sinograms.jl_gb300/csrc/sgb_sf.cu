@@ -30,8 +30,15 @@
 //     lies within the rows' range); per line it computes into shared memory the footprints of the
 //     pixels the chunk's wedge of rays can reach, and each bin sums the few pixels its own wedge
 //     reaches.  Deterministic, no atomics;
-//   * back: one thread per pixel, over the views and the bins its footprint covers.
+//   * back: one thread per pixel, over the views and the bins its footprint covers; small images split the
+//     views over a cluster, summed in rank order;
+//   * an element costs some 30 instructions, and under the scan's symmetry (scan_slots) a pixel's images
+//     have the same elements in the views that see them alike, at the same bins or at those mirrored about
+//     the detector's centre.  So the forward kernel sums a view's bins over the image together with the
+//     bins of the views that are its images, over the image's images, and the back-projector takes a pixel
+//     with its images: each element is evaluated once for two or four.
 // Plans compute the per-view constants and the boundary-ray table once, in FP64 on the device.
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -39,6 +46,7 @@
 
 #include "sgb_common.cuh"
 #include "sgb_host.h"
+#include "sgb_kernels.cuh"
 
 namespace sgb {
 
@@ -48,7 +56,8 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr int kFwdThreads = 128;                  // threads per forward CTA
 constexpr int kFwdBpt = 2;                        // adjacent detector bins per forward thread
 constexpr int kFwdBins = kFwdThreads * kFwdBpt;   // detector bins per forward CTA
-constexpr int kFwdCap = 384;                      // footprints per line pass of a forward CTA
+template <int NS>  // footprints per line pass of a forward CTA
+constexpr int kFwdCap = NS == 1 ? 384 : 256;
 constexpr int kBackTx = 32, kBackTy = 8;
 constexpr int kViewChunk = 64;  // views staged in shared memory per back-projector pass
 constexpr float kRangeEps = 0.01f;  // pixel-index margin of the candidate ranges (FP32 rounding)
@@ -76,8 +85,15 @@ static_assert(sizeof(SfView) == 80, "SfView layout");
 struct SfArgs {
     int nb, na, nx, ny;
     int splits;  // forward: the image lines are split over this many CTAs per (view, chunk of bins)
+    int gsplit;  // back: CTAs of a cluster that share a tile's views
+    int nrep;    // forward: views that are not images of others
+    ScanSlots sym;
     float wb, ax, ay, axy, hx, hy;
 };
+
+// A view and its images in the slots: entry j is slot j's view, kSfRev if its bins run the other way,
+// kSfDup if an earlier slot has the same view.
+constexpr int kSfRev = 1 << 30, kSfDup = 1 << 29, kSfView = kSfDup - 1;
 
 // One pixel's footprint in one view, relative to uc.
 struct SfRec {
@@ -264,18 +280,45 @@ __global__ void sf_setup_rays(SfGeo G, const double *betas, const SfView *views,
 }
 
 // ------------------------------------------------------------------- forward
-template <int GEO>
+// The model's image (mask applied) and its transpose: a pass reads consecutive pixels of a line, which
+// lie along x or along y.
+__global__ void sf_image_kernel(const float *__restrict__ image, const uint8_t *__restrict__ mask, int nx, int ny,
+                                float *__restrict__ out, float *__restrict__ outt) {
+    __shared__ float tile[32][33];
+    const int x = blockIdx.x * 32 + threadIdx.x, y0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int y = y0 + r;
+        if (x >= nx || y >= ny) continue;
+        const size_t n = x + (size_t)nx * y;
+        const float v = mask && !mask[n] ? 0.f : image[n];
+        out[n] = v;
+        tile[r][threadIdx.x] = v;
+    }
+    __syncthreads();
+    const int y = y0 + threadIdx.x;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int c = blockIdx.x * 32 + r;
+        if (c < nx && y < ny) outt[y + (size_t)ny * c] = tile[threadIdx.x][r];
+    }
+}
+
+template <int GEO, int NS>
 __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const SfView *__restrict__ views,
                                                                  const float2 *__restrict__ rays,
                                                                  const float *__restrict__ xcs,
                                                                  const float *__restrict__ ycs,
                                                                  const float *__restrict__ image,
-                                                                 const uint8_t *__restrict__ mask,
+                                                                 const float *__restrict__ imaget,
+                                                                 const int4 *__restrict__ images,
                                                                  float *__restrict__ sino) {
-    __shared__ float4 s0[2][kFwdCap];  // uc, d0, d1, d2
-    __shared__ float4 s1[2][kFwdCap];  // d3, hr01, hr23, c3 (fan beams)
-    __shared__ float2 s2[2][kFwdCap];  // h, pixel value
-    const int v = blockIdx.y, tid = threadIdx.x;
+    constexpr int CAP = kFwdCap<NS>;
+    __shared__ float4 s0[2][CAP];                // uc, d0, d1, d2
+    __shared__ float4 s1[GEO != 0 ? 2 : 1][CAP];  // d3, hr01, hr23, c3 (fan beams)
+    __shared__ float s2[2][CAP];                 // h
+    __shared__ float s3[2][NS][CAP];             // the pixel's value, and its images'
+    const int4 im = images[blockIdx.y];
+    const int iv[4] = {im.x, im.y, im.z, im.w};
+    const int v = iv[0], tid = threadIdx.x;
     const int k0 = blockIdx.x * kFwdBins, kend = min(k0 + kFwdBins, A.nb);
     const int ka = k0 + kFwdBpt * tid, kb = min(ka + kFwdBpt, A.nb);  // this thread's bins [ka, kb)
     const SfView V = views[v];
@@ -290,66 +333,129 @@ __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const
     // boundaries of bins ka and ka + 1 (exact in FP32, as the back-projector forms them)
     const float e0 = (float)ka - 0.5f, e1 = (float)ka + 0.5f, e2 = (float)(ka + 1) + 0.5f;
     const int per = (nln + A.splits - 1) / A.splits, jb = blockIdx.z * per, je = min(nln, jb + per);
-    float acc0 = 0.f, acc1 = 0.f;
-    int buf = 0;
-    for (int j = jb; j < je; j++) {
-        const float lc = lcs[j], L0 = lc - hl, L1 = lc + hl;
-        int ia, ib;
-        sf_range(cl, ch, L0, L1, nal, ia, ib);
-        if (ia > ib) continue;  // same for the whole CTA
-        int qa = 0, qb = -1;
-        if (active) sf_range(bl, bh, L0, L1, nal, qa, qb);
-        for (int p0 = ia; p0 <= ib; p0 += kFwdCap) {
-            const int p1 = min(ib, p0 + kFwdCap - 1);
-            for (int t = tid; t <= p1 - p0; t += kFwdThreads) {
-                const int i = p0 + t;
-                const int px = rows ? i : j, py = rows ? j : i;
-                const size_t n = (size_t)px + (size_t)A.nx * py;
-                float val = __ldg(image + n);
-                if (mask && !mask[n]) val = 0.f;
-                const SfRec r = sf_pixel<GEO>(V, A, __ldg(xcs + px), __ldg(ycs + py));
-                s0[buf][t] = make_float4(r.uc, r.d0, r.d1, r.d2);
-                if (GEO != 0) s1[buf][t] = make_float4(r.d3, r.hr01, r.hr23, r.c3);
-                s2[buf][t] = make_float2(r.h, val);
-            }
-            __syncthreads();
-            const int ta = max(qa, p0), tb = min(qb, p1);
-            for (int i = ta; i <= tb; i++) {
-                const int t = i - p0;
-                const float4 a0 = s0[buf][t];
-                const float2 a2 = s2[buf][t];
-                SfRec r;
-                r.uc = a0.x;
-                if (GEO == 0) {
-                    r.d0 = V.p0;
-                    r.d1 = V.p1;
-                    r.d2 = V.p2;
-                    r.d3 = V.p3;
-                    r.hr01 = V.phr01;
-                    r.hr23 = V.phr23;
-                    r.c3 = V.pc3;
-                } else {
-                    const float4 a1 = s1[buf][t];
-                    r.d0 = a0.y;
-                    r.d1 = a0.z;
-                    r.d2 = a0.w;
-                    r.d3 = a1.x;
-                    r.hr01 = a1.y;
-                    r.hr23 = a1.z;
-                    r.c3 = a1.w;
-                }
-                const float g0 = sf_cdf(__fsub_rn(e0, r.uc), r), g1 = sf_cdf(__fsub_rn(e1, r.uc), r);
-                const float g2 = sf_cdf(__fsub_rn(e2, r.uc), r);
-                acc0 = __fmaf_rn(__fmul_rn(a2.x, __fsub_rn(g1, g0)), a2.y, acc0);
-                acc1 = __fmaf_rn(__fmul_rn(a2.x, __fsub_rn(g2, g1)), a2.y, acc1);
-            }
-            buf ^= 1;
+    float acc0[NS] = {}, acc1[NS] = {};
+    // A pass is at most CAP pixels of a line: [p0, p1] of line j, whose wedge ends at ib.  The next
+    // pass's values are requested and its footprints computed while the current one is summed: one
+    // barrier per pass, and the loads' latency lies behind the sums.
+    struct Pass {
+        int j, ib, p0, p1, qa, qb;
+    };
+    auto lines = [&](Pass &q) {  // the first line from q.j on with pixels
+        for (; q.j < je; q.j++) {
+            const float lc = lcs[q.j], L0 = lc - hl, L1 = lc + hl;
+            sf_range(cl, ch, L0, L1, nal, q.p0, q.ib);
+            if (q.p0 > q.ib) continue;  // same for the whole CTA
+            q.p1 = min(q.ib, q.p0 + CAP - 1);
+            q.qa = 0;
+            q.qb = -1;
+            if (active) sf_range(bl, bh, L0, L1, nal, q.qa, q.qb);
+            return;
         }
+    };
+    auto advance = [&](Pass q) {
+        if (q.p1 < q.ib) {
+            q.p0 = q.p1 + 1;
+            q.p1 = min(q.ib, q.p0 + CAP - 1);
+            return q;
+        }
+        q.j++;
+        lines(q);
+        return q;
+    };
+    constexpr int NT = (CAP + kFwdThreads - 1) / kFwdThreads;  // a thread's pixels of a pass
+    float vals[NT][NS];
+    // slot s's values along line j: src[s] + ls[s] j + is[s] i, consecutive in memory
+    const float *src[NS];
+    int ls[NS], is[NS];
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        const int f = A.sym.slot[s].map;
+        const bool along_x = rows != ((f & 4) != 0);
+        is[s] = f & (along_x ? 1 : 2) ? -1 : 1;
+        const int pitch = along_x ? A.nx : A.ny, nl = along_x ? A.ny : A.nx;
+        const bool back = f & (along_x ? 2 : 1);
+        ls[s] = back ? -pitch : pitch;
+        src[s] = (along_x ? image : imaget) + (is[s] < 0 ? pitch - 1 : 0) + (back ? (size_t)pitch * (nl - 1) : 0);
+    }
+    auto request = [&](const Pass &q) {
+#pragma unroll
+        for (int u = 0; u < NT; u++) {
+            const int i = q.p0 + tid + u * kFwdThreads;
+            if (q.j >= je || i > q.p1) continue;
+#pragma unroll
+            for (int s = 0; s < NS; s++) vals[u][s] = __ldg(src[s] + (ptrdiff_t)ls[s] * q.j + is[s] * i);
+        }
+    };
+    auto fill = [&](const Pass &q, int buf) {
+#pragma unroll
+        for (int u = 0; u < NT; u++) {
+            const int t = tid + u * kFwdThreads, i = q.p0 + t;
+            if (q.j >= je || i > q.p1) continue;
+            const int px = rows ? i : q.j, py = rows ? q.j : i;
+            const SfRec r = sf_pixel<GEO>(V, A, __ldg(xcs + px), __ldg(ycs + py));
+            s0[buf][t] = make_float4(r.uc, r.d0, r.d1, r.d2);
+            if (GEO != 0) s1[buf][t] = make_float4(r.d3, r.hr01, r.hr23, r.c3);
+            s2[buf][t] = r.h;
+#pragma unroll
+            for (int s = 0; s < NS; s++) s3[buf][s][t] = vals[u][s];
+        }
+    };
+    Pass cur{jb, 0, 0, 0, 0, -1};
+    lines(cur);
+    request(cur);
+    fill(cur, 0);
+    for (int buf = 0; cur.j < je; buf ^= 1) {
+        const Pass nxt = advance(cur);
+        __syncthreads();
+        request(nxt);
+        const int ta = max(cur.qa, cur.p0), tb = min(cur.qb, cur.p1);
+        for (int i = ta; i <= tb; i++) {
+            const int t = i - cur.p0;
+            const float4 a0 = s0[buf][t];
+            const float h = s2[buf][t];
+            SfRec r;
+            r.uc = a0.x;
+            if (GEO == 0) {
+                r.d0 = V.p0;
+                r.d1 = V.p1;
+                r.d2 = V.p2;
+                r.d3 = V.p3;
+                r.hr01 = V.phr01;
+                r.hr23 = V.phr23;
+                r.c3 = V.pc3;
+            } else {
+                const float4 a1 = s1[buf][t];
+                r.d0 = a0.y;
+                r.d1 = a0.z;
+                r.d2 = a0.w;
+                r.d3 = a1.x;
+                r.hr01 = a1.y;
+                r.hr23 = a1.z;
+                r.c3 = a1.w;
+            }
+            const float g0 = sf_cdf(__fsub_rn(e0, r.uc), r), g1 = sf_cdf(__fsub_rn(e1, r.uc), r);
+            const float g2 = sf_cdf(__fsub_rn(e2, r.uc), r);
+            const float w0 = __fmul_rn(h, __fsub_rn(g1, g0)), w1 = __fmul_rn(h, __fsub_rn(g2, g1));
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                const float val = s3[buf][s][t];
+                acc0[s] = __fmaf_rn(w0, val, acc0[s]);
+                acc1[s] = __fmaf_rn(w1, val, acc1[s]);
+            }
+        }
+        fill(nxt, buf ^ 1);
+        cur = nxt;
     }
     // splits > 1: partial sums, added in split order by sf_sum_splits
-    float *row = sino + (size_t)A.nb * (v + (size_t)A.na * blockIdx.z);
-    if (active) row[ka] = acc0;
-    if (ka + 1 < A.nb) row[ka + 1] = acc1;
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        if (iv[s] & kSfDup) continue;
+        const int ka1 = ka + 1, vs = iv[s] & kSfView;
+        const bool rev = iv[s] & kSfRev;
+        float *row = sino + (size_t)A.nb * (vs + (size_t)A.na * blockIdx.z);
+        if (active) row[rev ? A.nb - 1 - ka : ka] = acc0[s];
+        if (ka1 < A.nb) row[rev ? A.nb - 1 - ka1 : ka1] = acc1[s];
+    }
 }
 
 __global__ void sf_sum_splits(const float *__restrict__ part, int splits, long long n, float *__restrict__ sino) {
@@ -361,27 +467,36 @@ __global__ void sf_sum_splits(const float *__restrict__ part, int splits, long l
 }
 
 // ------------------------------------------------------------------- back
-template <int GEO>
+template <int GEO, int NS>
 __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, const SfView *__restrict__ views,
                                                                    const float *__restrict__ xcs,
                                                                    const float *__restrict__ ycs,
                                                                    const float *__restrict__ sino,
                                                                    const uint8_t *__restrict__ mask,
+                                                                   const int4 *__restrict__ images,
                                                                    float *__restrict__ image) {
     __shared__ SfView sv[kViewChunk];
-    const int tid = threadIdx.x + kBackTx * threadIdx.y;
+    __shared__ int4 si[kViewChunk];
+    __shared__ float part[NS][kBackTx * kBackTy];
+    const int tid = threadIdx.x + kBackTx * threadIdx.y, rank = blockIdx.z;
     const int px = blockIdx.x * kBackTx + threadIdx.x, py = blockIdx.y * kBackTy + threadIdx.y;
-    const bool in = px < A.nx && py < A.ny;
-    const size_t n = in ? (size_t)px + (size_t)A.nx * py : 0;
-    const bool on = in && (!mask || mask[n]);
-    const float xc = in ? xcs[px] : 0.f, yc = in ? ycs[py] : 0.f;
-    float acc = 0.f;
-    for (int v0 = 0; v0 < A.na; v0 += kViewChunk) {
-        const int nv = min(kViewChunk, A.na - v0);
+    size_t n[NS];
+    bool own[NS], on = false;  // slot s's pixel is this thread's; one of them is in the model
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        own[s] = slot_pixel(A.sym, A.nx, A.ny, s, px, py, &n[s]);
+        on |= own[s] && (!mask || mask[n[s]]);
+    }
+    const float xc = px < A.nx ? xcs[px] : 0.f, yc = py < A.ny ? ycs[py] : 0.f;
+    const int va = (int)((long long)A.na * rank / A.gsplit), vb = (int)((long long)A.na * (rank + 1) / A.gsplit);
+    float acc[NS] = {};
+    for (int v0 = va; v0 < vb; v0 += kViewChunk) {
+        const int nv = min(kViewChunk, vb - v0);
         __syncthreads();
         const int *src = reinterpret_cast<const int *>(views + v0);
         int *dst = reinterpret_cast<int *>(sv);
         for (int t = tid; t < nv * (int)(sizeof(SfView) / 4); t += kBackTx * kBackTy) dst[t] = __ldg(src + t);
+        if (tid < nv) si[tid] = images[v0 + tid];
         __syncthreads();
         if (!on) continue;
         for (int vv = 0; vv < nv; vv++) {
@@ -390,16 +505,90 @@ __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, con
             const int kf = max(0, (int)ceilf(fminf(fmaxf(lo, -1.f), (float)A.nb)));
             const int kl = min(A.nb - 1, (int)floorf(fminf(fmaxf(hi, -1.f), (float)A.nb)));
             if (kf > kl) continue;
-            const float *srow = sino + (size_t)A.nb * (v0 + vv);
+            const int4 im = si[vv];
+            const int iv[4] = {im.x, im.y, im.z, im.w};
+            const float *row[NS];
+            int step[NS];
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                step[s] = iv[s] & kSfRev ? -1 : 1;
+                row[s] = sino + (size_t)A.nb * (iv[s] & kSfView) + (iv[s] & kSfRev ? A.nb - 1 - kf : kf);
+            }
             float gprev = sf_cdf(__fsub_rn((float)kf - 0.5f, r.uc), r);
             for (int k = kf; k <= kl; k++) {
                 const float g = sf_cdf(__fsub_rn((float)k + 0.5f, r.uc), r);
-                acc = __fmaf_rn(__fmul_rn(r.h, __fsub_rn(g, gprev)), __ldg(srow + k), acc);
+                const float w = __fmul_rn(r.h, __fsub_rn(g, gprev));
+#pragma unroll
+                for (int s = 0; s < NS; s++) {
+                    acc[s] = __fmaf_rn(w, __ldg(row[s]), acc[s]);
+                    row[s] += step[s];
+                }
                 gprev = g;
             }
         }
     }
-    if (in) image[n] = on ? acc : 0.f;
+    if (A.gsplit == 1) {
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            if (own[s]) image[n[s]] = !mask || mask[n[s]] ? acc[s] : 0.f;
+        return;
+    }
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+    for (int s = 0; s < NS; s++) part[s][tid] = acc[s];
+    cl.sync();
+    // each rank finishes its share of the slots' pixels, adding the ranks in order
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        if ((tid / 32 + s) % A.gsplit != rank || !own[s]) continue;
+        float v = 0.f;
+        for (int q = 0; q < A.gsplit; q++) v += cl.map_shared_rank(&part[s][tid], q)[0];
+        image[n[s]] = !mask || mask[n[s]] ? v : 0.f;
+    }
+    cl.sync();  // peers' shared memory stays alive until every rank has read it
+}
+
+template <int GEO, int NS>
+int sf_launch_back(const SfArgs &A, const SfView *views, const float *xcs, const float *ycs, const float *sino,
+                   const uint8_t *mask, const int4 *images, float *image, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((A.sym.hx + kBackTx - 1) / kBackTx, (A.sym.hy + kBackTy - 1) / kBackTy, A.gsplit);
+    cfg.blockDim = dim3(kBackTx, kBackTy);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = A.gsplit;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, sf_back_kernel<GEO, NS>, A, views, xcs, ycs, sino, mask, images, image);
+    if (e != cudaSuccess) {
+        set_error("sf_back_kernel: launch failed: %s", cudaGetErrorString(e));
+        return SGB_ERR_CUDA;
+    }
+    return after_launch("sf_back_kernel");
+}
+
+// One slot count of a direction, for the plan's geometry kind.
+template <int NS>
+int sf_launch(int kind, bool forward, const SfArgs &A, const SfView *views, const float2 *rays, const float *xcs,
+              const float *ycs, const float *src, const float *srct, const uint8_t *mask, const int4 *reps, const int4 *images, float *dst,
+              cudaStream_t st) {
+    if (!forward) {
+        if (kind == SGB_PAR) return sf_launch_back<0, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
+        if (kind == SGB_ARC) return sf_launch_back<1, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
+        return sf_launch_back<2, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
+    }
+    const dim3 grid((A.nb + kFwdBins - 1) / kFwdBins, A.nrep, A.splits);
+    if (kind == SGB_PAR)
+        sf_project_kernel<0, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
+    else if (kind == SGB_ARC)
+        sf_project_kernel<1, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
+    else
+        sf_project_kernel<2, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
+    return after_launch("sf_project_kernel");
 }
 
 }  // namespace
@@ -413,7 +602,8 @@ using namespace sgb;
 struct sgb_sf_plan {
     SfGeo G{};
     SfArgs A{};
-    DevBuf betas, views, rays, axes, mask, din, dout, part;
+    DevBuf betas, views, rays, axes, mask, din, dout, part, img;
+    DevBuf images;  // every view's images (na), then the representative views' (nrep)
     const uint8_t *mask_dev = nullptr;
 };
 
@@ -469,14 +659,14 @@ int sf_geometry(const sgb_sino_geom *rg, const sgb_image_geom *ig, SfGeo *G) {
 }
 
 // Line splits of the forward projector: enough CTAs for about two resident waves of four-warp
-// CTAs (16 per SM), at most 16 and at least 8 image lines per CTA.
-int sf_default_splits(const SfGeo &G) {
+// CTAs (16 per SM), at most 32 and at least 8 image lines per CTA.
+int sf_default_splits(const SfGeo &G, int nrep) {
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
-    const long long ctas = (long long)((G.nb + kFwdBins - 1) / kFwdBins) * G.na;
+    const long long ctas = (long long)((G.nb + kFwdBins - 1) / kFwdBins) * nrep;
     const long long want = 2LL * 16 * std::max(sms, 1);
-    int s = (int)std::min<long long>(16, std::max<long long>(1, (want + ctas - 1) / ctas));
+    int s = (int)std::min<long long>(32, std::max<long long>(1, (want + ctas - 1) / ctas));
     const int lines = std::max(G.nx, G.ny);
     while (s > 1 && lines / s < 8) s--;
     return s;
@@ -496,36 +686,32 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
     const float *xcs = P->axes.as<float>(), *ycs = xcs + G.nx;
     const SfView *views = P->views.as<SfView>();
     const float *src = static_cast<const float *>(in_dev);
+    const int4 *images = P->images.as<int4>();
+    auto run = [&](bool fwd, float *dst) {
+        const float2 *rays = P->rays.as<float2>();
+        auto go = P->A.sym.ns == 4 ? sf_launch<4> : (P->A.sym.ns == 2 ? sf_launch<2> : sf_launch<1>);
+        return go(G.kind, fwd, P->A, views, rays, xcs, ycs, fwd ? P->img.as<float>() : src, P->img.as<float>() + nimg, P->mask_dev,
+                  images + G.na, images, dst, st);
+    };
     if (forward) {
         const int splits = P->A.splits;
-        const dim3 grid((G.nb + kFwdBins - 1) / kFwdBins, G.na, splits);
         static_assert(kFwdBpt == 2, "sf_project_kernel accumulates two bins per thread");
-        const float2 *rays = P->rays.as<float2>();
         float *dst = out_dev;
         if (splits > 1) {
             SGB_TRY(P->part.reserve(sizeof(float) * nsino * splits));
             dst = P->part.as<float>();
         }
-        if (G.kind == SGB_PAR)
-            sf_project_kernel<0><<<grid, kFwdThreads, 0, st>>>(P->A, views, rays, xcs, ycs, src, P->mask_dev, dst);
-        else if (G.kind == SGB_ARC)
-            sf_project_kernel<1><<<grid, kFwdThreads, 0, st>>>(P->A, views, rays, xcs, ycs, src, P->mask_dev, dst);
-        else
-            sf_project_kernel<2><<<grid, kFwdThreads, 0, st>>>(P->A, views, rays, xcs, ycs, src, P->mask_dev, dst);
-        SGB_TRY(after_launch("sf_project_kernel"));
+        SGB_TRY(P->img.reserve(sizeof(float) * 2 * nimg));
+        sf_image_kernel<<<dim3((G.nx + 31) / 32, (G.ny + 31) / 32), dim3(32, 8), 0, st>>>(
+            src, P->mask_dev, G.nx, G.ny, P->img.as<float>(), P->img.as<float>() + nimg);
+        SGB_TRY(after_launch("sf_image_kernel"));
+        SGB_TRY(run(true, dst));
         if (splits > 1) {
             sf_sum_splits<<<(unsigned)((nsino + 255) / 256), 256, 0, st>>>(dst, splits, (long long)nsino, out_dev);
             SGB_TRY(after_launch("sf_sum_splits"));
         }
     } else {
-        const dim3 grid((G.nx + kBackTx - 1) / kBackTx, (G.ny + kBackTy - 1) / kBackTy), block(kBackTx, kBackTy);
-        if (G.kind == SGB_PAR)
-            sf_back_kernel<0><<<grid, block, 0, st>>>(P->A, views, xcs, ycs, src, P->mask_dev, out_dev);
-        else if (G.kind == SGB_ARC)
-            sf_back_kernel<1><<<grid, block, 0, st>>>(P->A, views, xcs, ycs, src, P->mask_dev, out_dev);
-        else
-            sf_back_kernel<2><<<grid, block, 0, st>>>(P->A, views, xcs, ycs, src, P->mask_dev, out_dev);
-        SGB_TRY(after_launch("sf_back_kernel"));
+        SGB_TRY(run(false, out_dev));
     }
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(out, out_dev, nout * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -574,7 +760,32 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
     A.axy = (float)std::fabs(G.dx * G.dy);
     A.hx = (float)(0.5 * std::fabs(G.dx));
     A.hy = (float)(0.5 * std::fabs(G.dy));
-    A.splits = sf_default_splits(G);
+    A.sym = scan_slots(rg->kind, G.na, G.nx, G.ny, 2 * G.wb == G.nb - 1.0, G.so == 0, rg->orbit, rg->orbit_start, ig->deltas,
+                       ig->offsets, false);
+    // every view's images, and those of the views that no earlier one's images include
+    std::vector<int4> images(G.na), reps;
+    std::vector<char> seen(G.na, 0);
+    for (int v = 0; v < G.na; v++) {
+        int e[4] = {v, 0, 0, 0};
+        for (int j = 1; j < A.sym.ns; j++) {
+            bool rev;
+            const int u = slot_view(A.sym, G.na, j, v, &rev);
+            e[j] = u | (rev ? kSfRev : 0);
+            for (int i = 0; i < j; i++)
+                if ((e[i] & kSfView) == u) e[j] |= kSfDup;
+        }
+        images[v] = make_int4(e[0], e[1], e[2], e[3]);
+        if (!seen[v]) reps.push_back(images[v]);
+        for (int j = 0; j < A.sym.ns; j++) seen[e[j] & kSfView] = 1;
+    }
+    A.nrep = (int)reps.size();
+    images.insert(images.end(), reps.begin(), reps.end());
+    SGB_TRY(P->images.reserve(sizeof(int4) * images.size()));
+    SGB_CUDA(cudaMemcpyAsync(P->images.p, images.data(), sizeof(int4) * images.size(), cudaMemcpyHostToDevice, st));
+    A.splits = sf_default_splits(G, A.nrep);
+    // back: about four CTAs of 256 pixels per SM, at least 8 views each
+    const long long tiles = (long long)((A.sym.hx + kBackTx - 1) / kBackTx) * ((A.sym.hy + kBackTy - 1) / kBackTy);
+    A.gsplit = (int)std::max<long long>(1, std::min<long long>({8, G.na / 8, (4LL * std::max(1, num_sms()) + tiles / 2) / tiles}));
     SGB_TRY(P->views.reserve(sizeof(SfView) * G.na));
     SGB_TRY(P->rays.reserve(sizeof(float2) * (size_t)G.na * (G.nb + 1)));
     sf_setup_views<<<(G.na + 127) / 128, 128, 0, st>>>(G, P->betas.as<double>(), P->views.as<SfView>());
