@@ -10,11 +10,12 @@
 // affine function of the pixel index: rowm[c] = r0 + c * delta.  The kernels use that
 // closed form instead of a table.  The interpolated prefix integral of a row at a mapped
 // point is F(q) = delta * (sum_{c<floor q} val[c] + frac(q) val[floor q]), q = (u-r0)/delta,
-// clamped to [0, nPix] (Flat extrapolation).  The forward projector takes the reference's
-// |diff| of F at consecutive detector boundaries from a warp-level prefix scan kept in
-// two-float (hi + lo) arithmetic, so nearby prefix values subtract without losing FP32
-// accuracy.  The back-projector is the transpose: a warp-level two-float scan of each view's
-// detector-bin integrals gives the detector prefix integral at the knots, and each pixel's
+// clamped to [0, nPix] (Flat extrapolation).  The forward projector forms the reference's
+// |diff| of F at consecutive detector boundaries from the pixels between them directly, or, where
+// a bin covers many, from a warp-level prefix scan kept in two-float (hi + lo) arithmetic, so
+// nearby prefix values subtract without losing FP32 accuracy.  The back-projector is the
+// transpose: a block-wide two-float scan of each view's detector-bin integrals gives the detector
+// prefix integral at the knots, and each pixel's
 // value is |G(u1) - G(u0)| of that prefix interpolated at the pixel's two mapped boundaries
 // (:196-205).  Both are exactly the reference's quantity.  FP64 is kept for the per-view and
 // per-row geometry (trig, boundary mapping); the per-sample work is FP32.
@@ -29,6 +30,7 @@
 // the first view's row block once more without the y-axis transpose.
 #include <algorithm>
 
+#include "sgb_async.cuh"
 #include "sgb_common.cuh"
 #include "sgb_kernels.cuh"
 
@@ -40,6 +42,18 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr int kWarps = 8;
 constexpr int kThreads = 32 * kWarps;
 constexpr int kStageU = 8;  // phantom loads per thread in flight while a row block is staged
+
+__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dev::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dev::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 struct ViewInfo {
     double rtx, rty;
@@ -446,25 +460,199 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 }
 
+// The same projection without prefixes, for bins that cover few pixels.  A bin between mapped
+// boundaries q0, q1 (in pixels, c0 = floor(q0) <= c1 = floor(q1)) integrates
+// (c1 - q0) val[c0] + (q1 - c1) val[c1] when c1 <= c0 + 1, and when c1 == c0 the same expression
+// still gives (q1 - q0) val[c0]: no prefix integral and no difference of large sums.  Bins that
+// cover more pixels add the whole ones between in a loop, which a warp enters only when one of its
+// bins does.  A lane holds kDirBins consecutive bins of a group of 31 x kDirBins and takes its last
+// boundary from the next lane: a boundary is evaluated once but for 1 in 32.
+//
+// A warp has whole rows, or every wb-th of their groups when there are more than kDirGroups: the
+// bins that cover several pixels lie together at one end of a view, and a split of the bins into
+// ranges left the other warps waiting for that end's (121 us at 512^2 x 888 x 90 views, this one
+// 72).  Its sums stay in registers over the CTA's rows.  The prefix form took 106 us there: it
+// spends about as much on each staged row's scan as on its bins.  Bound by issue (64 % of the
+// slots; 48 million instructions, of which staging is an eighth).
+constexpr int kDirRows = 8;                // rows per stage
+constexpr int kDirBins = 4;                // bins per lane and group
+constexpr int kDirGroup = 31 * kDirBins;  // bins per group
+constexpr int kDirGroups = 4;              // groups per warp
+
+// staged row pitch: 4 mod 32 words, so the transposing stores (8 rows x 4 columns a warp) spread
+// over the banks
+__host__ __device__ __forceinline__ int direct_pitch(int nPix) { return (nPix + 1 + 27) / 32 * 32 + 4; }
+
+__global__ void __launch_bounds__(kThreads, 4)
+    bdd_project_direct_kernel(BddArgs G, const ViewInfo *info, const float *detm, const float *L, const float4 *rmap,
+                              const float *__restrict__ phantom, float *sino, int rows_per_cta, int wb) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int nPix = G.nPix, nDet = G.nDet, p = blockIdx.x;
+    const int pitch = direct_pitch(nPix);
+    float4 *rm = reinterpret_cast<float4 *>(smraw);             // 2 x kDirRows row maps
+    float4 *dms = rm + 2 * kDirRows;                             // kDirGroups x wb x 32: the lanes' boundaries
+    float *vw = reinterpret_cast<float *>(dms + kDirGroups * wb * 32);  // 2 x kDirRows x pitch values
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    const int axis = info[p].axis;
+    const float *dview = detm + (size_t)p * (nDet + 1);
+    const int sub = warp / wb, nsub = kWarps / wb;  // rows sub, sub + nsub, ... of a stage
+    const int z0 = blockIdx.z * wb * kDirGroups * kDirGroup;
+    const int ngroup = min(kDirGroups * wb, (nDet - z0 + kDirGroup - 1) / kDirGroup);  // of this CTA
+    for (int i = threadIdx.x; i < ngroup * 32; i += kThreads) {
+        const int k = z0 + (i / 32) * kDirGroup + (i % 32) * kDirBins;
+        dms[i] = make_float4(dview[min(k, nDet)], dview[min(k + 1, nDet)], dview[min(k + 2, nDet)],
+                             dview[min(k + 3, nDet)]);
+    }
+    float acc[kDirGroups][kDirBins];
+#pragma unroll
+    for (int g = 0; g < kDirGroups; g++)
+#pragma unroll
+        for (int i = 0; i < kDirBins; i++) acc[g][i] = 0.f;
+    if (threadIdx.x < 2 * kDirRows) vw[threadIdx.x * pitch + nPix] = 0.f;  // q = nPix reads it
+    const int r_begin = blockIdx.y * rows_per_cta, r_end = min(nPix, r_begin + rows_per_cta);
+    // x-case row r = phantom[r + nPix*c] (eight consecutive r per 32-byte sector); y-case
+    // (transposed and reversed, :67) row r = phantom[(nPix-1-c) + nPix*r]
+    auto stage = [&](int rb, int s) {
+        const int nr = min(kDirRows, r_end - rb);
+        float *dst = vw + s * kDirRows * pitch;
+        if (axis) {
+            const int j = threadIdx.x % kDirRows;
+            if (j < nr) {
+                const float *src = phantom + rb + j;
+                for (int c = threadIdx.x / kDirRows; c < nPix; c += kThreads / kDirRows)
+                    cp_async4(dst + j * pitch + c, src + (size_t)nPix * c);
+            }
+        } else if (warp < nr) {
+            const float *src = phantom + (size_t)nPix * (rb + warp) + (nPix - 1);
+            for (int c = lane; c < nPix; c += 32) cp_async4(dst + warp * pitch + c, src - c);
+        }
+        if (threadIdx.x < nr) cp_async16(rm + s * kDirRows + threadIdx.x, rmap + (size_t)p * nPix + rb + threadIdx.x);
+        cp_async_commit();
+    };
+    const float qmax = (float)nPix;
+    stage(r_begin, 0);
+    int s = 0;
+    for (int rb = r_begin; rb < r_end; rb += kDirRows, s ^= 1) {
+        if (rb + kDirRows < r_end) {
+            stage(rb + kDirRows, s ^ 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        const int nrows = min(kDirRows, r_end - rb);
+        for (int j = sub; j < nrows; j += nsub) {
+            const float4 m = rm[s * kDirRows + j];  // (r0, delta, 1 / delta, |delta|)
+            const float *vj = vw + (s * kDirRows + j) * pitch;
+#pragma unroll
+            for (int g = 0; g < kDirGroups; g++) {
+                const int gi = g * wb + warp % wb;
+                if (gi >= ngroup) break;  // uniform
+                const float4 d4 = dms[gi * 32 + lane];
+                const float dm[kDirBins] = {d4.x, d4.y, d4.z, d4.w};
+                float q[kDirBins + 1], c[kDirBins + 1], v[kDirBins + 1];
+#pragma unroll
+                for (int i = 0; i <= kDirBins; i++) {
+                    if (i < kDirBins) q[i] = fminf(fmaxf((dm[i] - m.x) * m.z, 0.f), qmax);
+                    else q[i] = __shfl_down_sync(full, q[0], 1);
+                    // floor(q) for 0 <= q <= nPix < 2^22 by the round-down add of 2^23
+                    const float t = __fadd_rd(q[i], 8388608.f);
+                    c[i] = t - 8388608.f;
+                    if (i < kDirBins) v[i] = vj[__float_as_int(t) - 0x4B000000];
+                    else v[i] = __shfl_down_sync(full, v[0], 1);
+                }
+                float a[kDirBins], wide = 0.f;
+#pragma unroll
+                for (int i = 0; i < kDirBins; i++) {
+                    const float e = fmaxf(c[i], c[i + 1]);
+                    wide = fmaxf(wide, fabsf(c[i + 1] - c[i]));
+                    a[i] = fmaf(e - q[i], v[i], (q[i + 1] - e) * v[i + 1]);
+                }
+                if (wide > 1.5f && lane < 31) {  // (lane 31 has one boundary only)
+                    // whole pixels between the boundaries' own, which the sum above has as the lower
+                    // one's value
+#pragma unroll
+                    for (int i = 0; i < kDirBins; i++) {
+                        const bool up = q[i] <= q[i + 1];
+                        const float vb = up ? v[i] : v[i + 1];
+                        const int hi = (int)fmaxf(c[i], c[i + 1]);
+                        float t = 0.f;
+                        for (int k = (int)fminf(c[i], c[i + 1]) + 1; k < hi; k++) t += vj[k] - vb;
+                        a[i] += up ? t : -t;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < kDirBins; i++) acc[g][i] = fmaf(fabsf(a[i]), m.w, acc[g][i]);  // :98-101
+            }
+        }
+        __syncthreads();
+    }
+    // the row subsets' sums, in order (the staged rows are done with)
+    float *red = vw;  // nsub x (ngroup x kDirGroup)
+    const int nb = ngroup * kDirGroup;
+#pragma unroll
+    for (int g = 0; g < kDirGroups; g++) {
+        const int gi = g * wb + warp % wb;
+        if (gi >= ngroup || lane == 31) break;
+#pragma unroll
+        for (int i = 0; i < kDirBins; i++) red[sub * nb + gi * kDirGroup + lane * kDirBins + i] = acc[g][i];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb && z0 + i < nDet; i += kThreads) {
+        float t = 0.f;
+        for (int w = 0; w < nsub; w++) t += red[w * nb + i];
+        atomicAdd(sino + p + (size_t)G.na * (z0 + i), t * L[(size_t)p * nDet + z0 + i]);  // :104
+    }
+}
+
 // ------------------------------------------------------------------ backward
-// words per warp of the back-projector's skewed pixel accumulators (pixel c at c + c / 16)
-__host__ __device__ __forceinline__ int back_acc_pitch(int nPix) { return nPix + nPix / 16 + 1; }
-// float4 slots of the swizzled knot table: nDet + 1 knots rounded up to whole groups of 8
-__host__ __device__ __forceinline__ int back_tab_slots(int nDet) { return (nDet + 1 + 7) / 8 * 8; }
+// The back-projector's table of one view, one contiguous block: the guess table (kCells + 1 pairs:
+// the fractional knot index at the start of each of kCells equal cells of the mapped axis, and its
+// rise over the cell), the knots K (ascending), the density of each bin, and the two-float prefix
+// at the knots.  The first two depend on the geometry only and are written at set-up.
+constexpr int kCells = 256;
+constexpr int kGuessFloats = 2 * (kCells + 2);  // a multiple of 4 floats
+__host__ __device__ __forceinline__ int back_knots(int nDet) { return (nDet + 1 + 3) / 4 * 4; }
+__host__ __device__ __forceinline__ int back_view_floats(int nDet) { return kGuessFloats + 4 * back_knots(nDet); }
+
+// Guess table of one view: entry i = (x_i, x_{i+1} - x_i), x_i the fractional knot index at
+// kfirst + i (klast - kfirst) / kCells.
+__device__ __forceinline__ float knot_index(const float4 *geo, int nDet, float u) {
+    int lo = 0, hi = nDet;  // K[lo] <= u < K[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (geo[mid].x <= u) lo = mid; else hi = mid;
+    }
+    const float w = geo[lo + 1].x - geo[lo].x;
+    return (float)lo + fminf(fmaxf((u - geo[lo].x) / w, 0.f), 1.f);
+}
+__global__ void __launch_bounds__(kThreads) bdd_guess_kernel(BddArgs G, const float4 *__restrict__ geo, float *tab) {
+    const int p = blockIdx.x, nDet = G.nDet;
+    const float4 *Gv = geo + (size_t)p * (nDet + 1);
+    float *T = tab + (size_t)p * back_view_floats(nDet);
+    const float k0 = Gv[0].x, h = (Gv[nDet].x - k0) / kCells;
+    for (int i = threadIdx.x; i <= kCells; i += kThreads) {
+        const float a = knot_index(Gv, nDet, fmaf((float)i, h, k0)), b = knot_index(Gv, nDet, fmaf((float)(i + 1), h, k0));
+        reinterpret_cast<float2 *>(T)[i] = make_float2(a, i < kCells ? b - a : 0.f);
+    }
+    for (int j = threadIdx.x; j <= nDet; j += kThreads) T[kGuessFloats + j] = Gv[j].x;
+}
 
 // The back-projector's per-call table: one CTA per view forms each bin's integral B[j] =
 // sino * (geometry factor) and density, in ascending knot order, and the two-float prefix of B
 // over the knots (integrate1D, :229-241, of the weighted sinogram, :196), by a block-wide scan:
 // each thread sums a contiguous run of bins, the runs' totals are scanned within each warp by
-// shuffles and across the warps through shared memory, in order.  T[j] = (K[j], density of bin
-// j, prefix hi, prefix lo), T[nDet] = (K[nDet], 0, total).
+// shuffles and across the warps through shared memory, in order.  Knot nDet has density 0 and the
+// total.
 __global__ void __launch_bounds__(kThreads) bdd_fill_prefix_kernel(BddArgs G, const float *__restrict__ sino,
-                                                                  const float4 *__restrict__ geo, float4 *tab) {
+                                                                  const float4 *__restrict__ geo, float *tab) {
     __shared__ float2 wtot[kWarps];
     const int p = blockIdx.x, nDet = G.nDet;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float4 *Gv = geo + (size_t)p * (nDet + 1);
-    float4 *T = tab + (size_t)p * (nDet + 1);
+    float *dens = tab + (size_t)p * back_view_floats(nDet) + kGuessFloats + back_knots(nDet);
+    float2 *pre = reinterpret_cast<float2 *>(dens + back_knots(nDet));
     const bool desc = Gv[nDet].w != 0.f;
     const int chunk = (nDet + kThreads - 1) / kThreads;
     const int j_begin = min(nDet, tid * chunk), j_end = min(nDet, j_begin + chunk);
@@ -494,94 +682,137 @@ __global__ void __launch_bounds__(kThreads) bdd_fill_prefix_kernel(BddArgs G, co
     for (int j = j_begin; j < j_end; j++) {
         const float s = sino[p + (size_t)G.na * (desc ? nDet - 1 - j : j)];
         const float4 g = Gv[j];
-        T[j] = make_float4(g.x, s * g.z, sh, sl);
+        dens[j] = s * g.z;
+        pre[j] = make_float2(sh, sl);
         two_sum_add(sh, sl, s * g.y);
     }
-    if (j_begin < nDet && j_end == nDet) T[nDet] = make_float4(Gv[nDet].x, 0.f, sh, sl);
-}
-
-// Shared-memory slot of knot j: XOR-swizzled within groups of 8 float4 (the 32 banks), so lanes
-// whose knots lie a fixed stride apart (each walks its own run of pixels) spread over the banks.
-__device__ __forceinline__ int tix(int j) { return j ^ ((j >> 3) & 7); }
-
-// G(u) = P[j] + (u - K[j]) * dens[j] for K[j] <= u <= K[j+1]: the detector prefix integral
-// linearly interpolated at u (:198-203), as (hi, lo).
-__device__ __forceinline__ void prefix_at(const float4 *T, int j, float u, float &gh, float &gl) {
-    const float4 t = T[tix(j)];
-    gh = t.z;
-    gl = fmaf(u - t.x, t.y, t.w);
-}
-
-// First knot interval of u: the largest j < nDet with K[j] <= u (0 below the first knot).
-__device__ __forceinline__ int knot_search(const float4 *T, int nDet, float u) {
-    int lo = 0, hi = nDet;  // K[lo] <= u < K[hi]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (T[tix(mid)].x <= u) lo = mid; else hi = mid;
+    if (j_begin < nDet && j_end == nDet) {
+        dens[nDet] = 0.f;
+        pre[nDet] = make_float2(sh, sl);
     }
-    return lo;
 }
 
 // Per image row and view: pixel c takes |G(u_{c+1}) - G(u_c)| (:205) at its mapped boundaries
-// u_c = r0 + c delta, clamped to the knots (Flat extrapolation, :199-201); the two-float prefix
-// keeps that difference accurate to FP32 relative to the pixel's own integral.  Each lane owns
-// a run of consecutive pixels and walks the knots along it, reusing G at the shared boundary.
-__global__ void __launch_bounds__(kThreads)
-    bdd_back_kernel(BddArgs G, const ViewInfo *info, const float4 *tab, const float4 *rmap, float *image,
-                    int views_per_cta) {
+// u_c = r0 + c delta, clamped to the knots (Flat extrapolation, :199-201), G the detector prefix
+// integral linearly interpolated (:198-203); the two-float prefix keeps that difference accurate
+// to FP32 relative to the pixel's own integral.
+//
+// A warp has one image row and up to kBackGroups groups of 31 pixels of it; lane c of a group
+// holds boundary c and takes the next lane's G.  The boundary's knot interval comes from the
+// view's guess table, put right against the knots themselves (rarely by more than nothing: the
+// table's linear steps are off by ~0.01 knots at 888 bins).  Neighbouring lanes read neighbouring
+// knots, and the pixel sums stay in registers over the CTA's views.  The views that map onto x are
+// taken first, then those that map onto y, which add to the transposed row (:210-212).
+//
+// Bound by issue (65 % of the slots) and shared loads (63 % of the wavefronts).  512^2 x 888 x 90
+// views: 70 us; a lane walking the knots along its own run of 16 pixels took 121, its knot reads
+// four to a bank and each waiting for the one before.
+constexpr int kBackGroups = 9, kBackBatch = 3;  // groups per warp, and of them at a time
+__global__ void __launch_bounds__(kThreads, 5)
+    bdd_back_kernel(BddArgs G, const ViewInfo *info, const float *tab, const float4 *rmap, float *image,
+                    int views_per_cta, int nchunk, int gpc, int nstage) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int nPix = G.nPix, nDet = G.nDet;
-    // per-warp pixel accumulators, skewed by one word per 16 pixels: a lane's run of pixels starts
-    // 16 pixels after its neighbour's, so the skew spreads the lanes over the banks
-    const int apitch = back_acc_pitch(nPix);
-    float4 *T = reinterpret_cast<float4 *>(smraw);                      // nDet+1 knots in tix order
-    float *accX = reinterpret_cast<float *>(T + back_tab_slots(nDet));  // kWarps x apitch
-    float *accY = accX + kWarps * apitch;
+    const int nPix = G.nPix, vf = back_view_floats(G.nDet);
+    const unsigned nDet = G.nDet;
+    float *sm = reinterpret_cast<float *>(smraw);  // nstage x vf
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * kWarps + warp;
-    for (int i = threadIdx.x; i < 2 * kWarps * apitch; i += kThreads) accX[i] = 0.f;
-    float *ax = accX + warp * apitch, *ay = accY + warp * apitch;
+    const unsigned full = 0xffffffffu;
+    const int unit = blockIdx.x * kWarps + warp, r = unit / nchunk;
+    const int c0 = (unit % nchunk) * gpc * 31 + lane;
+    const float cf = (float)c0;
     const int v_begin = blockIdx.y * views_per_cta, v_end = min(G.na, v_begin + views_per_cta);
-    const int per = (nPix + 31) / 32;  // contiguous pixels per lane
-    for (int p = v_begin; p < v_end; p++) {
-        __syncthreads();
-        for (int k = threadIdx.x; k <= nDet; k += kThreads) T[tix(k)] = tab[(size_t)p * (nDet + 1) + k];
-        __syncthreads();
-        if (r >= nPix) continue;
-        const ViewInfo vi = info[p];
-        const float4 rmv = rmap[(size_t)p * nPix + r];
-        const float r0 = rmv.x, delta = rmv.y;
-        const float kfirst = T[tix(0)].x, klast = T[tix(nDet)].x;
-        const int c_a = lane * per, c_b = min(nPix, c_a + per);
-        if (c_a >= c_b) continue;
-        float u = fminf(fmaxf(fmaf((float)c_a, delta, r0), kfirst), klast);
-        int j = knot_search(T, nDet, u);
-        float gh, gl;
-        prefix_at(T, j, u, gh, gl);
-        const bool up = delta > 0.f;  // the boundaries ascend (walk the knots forward) or descend
-        for (int c = c_a; c < c_b; c++) {
-            u = fminf(fmaxf(fmaf((float)(c + 1), delta, r0), kfirst), klast);
-            if (up)
-                while (j < nDet - 1 && T[tix(j + 1)].x <= u) j++;
-            else
-                while (j > 0 && T[tix(j)].x > u) j--;
-            float hh, hl;
-            prefix_at(T, j, u, hh, hl);
-            const float tmp = fabsf((hh - gh) + (hl - gl));  // :205
-            const int ca = c + (c >> 4);
-            if (vi.axis) ax[ca] += tmp;                       // :210
-            else ay[ca] += tmp;                               // :212
-            if (p == 0) ax[ca] += tmp;                        // aliasing of :139-140
-            gh = hh;
-            gl = hl;
+    auto stage = [&](int p, int s) {
+        const float4 *src = reinterpret_cast<const float4 *>(tab + (size_t)p * vf);
+        float4 *dst = reinterpret_cast<float4 *>(sm + s * vf);
+        for (int i = threadIdx.x; i < vf / 4; i += kThreads) cp_async16(dst + i, src + i);
+        cp_async_commit();
+    };
+    float acc[kBackGroups];
+#pragma unroll
+    for (int i = 0; i < kBackGroups; i++) acc[i] = 0.f;
+    for (int pass = 1; pass >= 0; pass--) {
+        // next view at or after p that this pass takes; view 0 also adds its untransposed row
+        // (aliasing of :139-140)
+        auto next = [&](int p) {
+            while (p < v_end && info[p].axis != pass && !(pass && p == 0)) p++;
+            return p;
+        };
+        int p = next(v_begin), s = 0;
+        if (p >= v_end) continue;  // uniform
+        stage(p, 0);
+        while (p < v_end) {
+            const int pn = next(p + 1);
+            if (nstage == 2 && pn < v_end) {
+                stage(pn, s ^ 1);
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
+            }
+            __syncthreads();
+            if (r < nPix) {
+                const float2 *guess = reinterpret_cast<const float2 *>(sm + s * vf);
+                const float *K = sm + s * vf + kGuessFloats, *dens = K + back_knots(nDet);
+                const float2 *pre = reinterpret_cast<const float2 *>(dens + back_knots(nDet));
+                const float4 rmv = rmap[(size_t)p * nPix + r];
+                const float r0 = rmv.x, delta = rmv.y;
+                const float kfirst = K[0], klast = K[nDet];
+                const float scale = klast > kfirst ? (float)kCells / (klast - kfirst) : 0.f;
+                const float wt = (pass && p == 0 && info[0].axis) ? 2.f : 1.f;
+#pragma unroll
+                for (int ib = 0; ib < kBackGroups; ib += kBackBatch) {
+                    if (ib >= gpc) break;  // uniform
+                    // floors by the round-down add of 2^23; the unsigned minima keep any index in
+                    // its table
+                    float u[kBackBatch], ka[kBackBatch], kb[kBackBatch];
+                    unsigned j[kBackBatch];
+                    bool off = false;
+#pragma unroll
+                    for (int i = 0; i < kBackBatch; i++) {
+                        u[i] = fminf(fmaxf(fmaf(cf + 31.f * (ib + i), delta, r0), kfirst), klast);
+                        const float x = (u[i] - kfirst) * scale, t = __fadd_rd(x, 8388608.f);
+                        const float2 e = guess[min(__float_as_uint(t) - 0x4B000000u, (unsigned)kCells)];
+                        const float y = fmaf(x - (t - 8388608.f), e.y, e.x);
+                        j[i] = min(__float_as_uint(__fadd_rd(y, 8388608.f)) - 0x4B000000u, nDet - 1);
+                        ka[i] = K[j[i]];
+                        kb[i] = K[j[i] + 1];
+                        off |= kb[i] <= u[i] || ka[i] > u[i];
+                    }
+                    if (off) {  // the largest j < nDet with K[j] <= u
+#pragma unroll
+                        for (int i = 0; i < kBackBatch; i++) {
+                            while (kb[i] <= u[i] && j[i] < nDet - 1) {
+                                j[i]++;
+                                ka[i] = kb[i];
+                                kb[i] = K[j[i] + 1];
+                            }
+                            while (ka[i] > u[i] && j[i] > 0) {
+                                j[i]--;
+                                ka[i] = K[j[i]];
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < kBackBatch; i++) {
+                        const float2 g = pre[j[i]];
+                        const float gh = g.x, gl = fmaf(u[i] - ka[i], dens[j[i]], g.y);
+                        const float hh = __shfl_down_sync(full, gh, 1), hl = __shfl_down_sync(full, gl, 1);
+                        acc[ib + i] = fmaf(fabsf((hh - gh) + (hl - gl)), wt, acc[ib + i]);  // :205
+                    }
+                }
+            }
+            __syncthreads();
+            if (nstage == 2) s ^= 1;
+            else if (pn < v_end) stage(pn, 0);
+            p = pn;
         }
-    }
-    __syncwarp();
-    if (r >= nPix) return;
-    for (int c = lane; c < nPix; c += 32) {
-        const float vx = ax[c + (c >> 4)], vy = ay[c + (c >> 4)];
-        if (vx != 0.f) atomicAdd(image + r + (size_t)nPix * c, vx);
-        if (vy != 0.f) atomicAdd(image + (nPix - 1 - c) + (size_t)nPix * r, vy);  // reverse(., 2)'
+#pragma unroll
+        for (int i = 0; i < kBackGroups; i++) {
+            const int c = c0 + 31 * i;
+            if (i < gpc && lane < 31 && r < nPix && c < nPix && acc[i] != 0.f)
+                atomicAdd(pass ? image + r + (size_t)nPix * c                       // :210
+                               : image + (nPix - 1 - c) + (size_t)nPix * r, acc[i]);  // :212, reverse(., 2)'
+            acc[i] = 0.f;
+        }
     }
 }
 
@@ -595,20 +826,61 @@ size_t project_bins_smem(const BddArgs &G) {
     return (sizeof(float2) + sizeof(float)) * (size_t)kWarps * (G.nPix + 1) + sizeof(RowMap) * kWarps +
            sizeof(float) * (size_t)(G.nDet + 1);
 }
-size_t back_smem(const BddArgs &G) {
-    return sizeof(float4) * (size_t)back_tab_slots(G.nDet) + sizeof(float) * 2 * (size_t)kWarps * back_acc_pitch(G.nPix);
+size_t project_direct_smem(const BddArgs &G, int wb) {
+    const size_t rows = 2 * kDirRows * (size_t)direct_pitch(G.nPix), sums = (size_t)kWarps * kDirGroups * kDirGroup;
+    return sizeof(float4) * (2 * kDirRows + 32 * (size_t)kDirGroups * wb) + sizeof(float) * std::max(rows, sums);
+}
+// The sizes this pair takes: the tables of one view with eight rows of both images, as the limit
+// has always been stated.
+bool back_fits(const BddArgs &G) {
+    return 16 * (size_t)((G.nDet + 1 + 7) / 8 * 8) + 8 * (size_t)kWarps * (G.nPix + G.nPix / 16 + 1) <= 220 * 1024;
+}
+// A mapped bin's width in pixels at the image centre; up to kDirectStep the direct kernel projects.
+// 90 views, us a projection, prefix and direct: 512^2, bins of 0.6 pixels 145 and 112, 1.0 131 and
+// 134, 2.0 120 and 107, 6.0 110 and 87; 1024^2, 0.6 494 and 312, 6.0 300 and 210; 256^2, 79 and 67,
+// 70 and 62.  Wider bins keep the prefix form: its differences stay good to FP32 however many pixels
+// lie in a bin.
+constexpr double kDirectStep = 6.0;
+double central_step(const BddArgs &G) { return G.dSize * G.DS0 / (G.DSD * G.pSize); }
+
+// Blocks per SM that `smem` bytes a block leave room for, at most `cap` (what the registers allow).
+int resident(size_t smem, int cap) { return std::max(1, std::min(cap, (int)(228 * 1024 / (smem + 1024)))); }
+
+// The split of n items over base x split CTAs, `res` of them at a time on an SM, with the least
+// time.  An SM issues at a fixed rate, so a wave takes as long as the items of its CTAs on one SM,
+// each CTA with one item more (its first stage and its atomic adds), and a last wave that is less
+// than 0.7 full no less than that: fewer warps leave issue slots idle.  Returns the items per CTA.
+int split_items(int n, long long base, int res) {
+    const long long sms = std::max(1, num_sms()), wave = sms * res;
+    int best = n;
+    double tb = 1e300;
+    for (int s = 1; s <= n; s++) {
+        const int per = (n + s - 1) / s;
+        const long long ctas = base * ((n + per - 1) / per), rest = ctas % wave;
+        const double last = rest ? std::max(0.7 * res, (double)((rest + sms - 1) / sms)) : 0.0;
+        const double t = ((double)(ctas / wave) * res + last) * (per + 1);
+        if (t < tb) {
+            tb = t;
+            best = per;
+        }
+        if (ctas > 16 * wave) break;
+    }
+    return best;
 }
 
 }  // namespace
 
 // Scratch layouts.  Forward: view records | detm (na x (nDet+1)) | L (na x nDet) | row maps
-// (na x nPix float4).  Back: view records | knot table | geometry table (na x (nDet+1) float4
-// each) | row maps.
+// (na x nPix float4).  Back: view records | per-view tables (guess, knots, densities, prefix) |
+// geometry table (na x (nDet+1) float4) | row maps.
 size_t proj_rowmap_offset(const BddArgs &G) {
     return (info_bytes(G.na) + sizeof(float) * ((size_t)G.na * (G.nDet + 1) + (size_t)G.na * G.nDet) + 15) / 16 * 16;
 }
+size_t back_geo_offset(const BddArgs &G) {
+    return info_bytes(G.na) + sizeof(float) * (size_t)G.na * back_view_floats(G.nDet);
+}
 size_t back_rowmap_offset(const BddArgs &G) {
-    return info_bytes(G.na) + 2 * sizeof(float4) * (size_t)G.na * (G.nDet + 1);
+    return back_geo_offset(G) + sizeof(float4) * (size_t)G.na * (G.nDet + 1);
 }
 
 size_t bdd_project_scratch(const BddArgs &G) {
@@ -654,6 +926,18 @@ int launch_bdd_project_main(const BddArgs &G, const float *phantom, float *sino,
     const float *L = detm + (size_t)G.na * (G.nDet + 1);
     const float4 *rmap = reinterpret_cast<const float4 *>(static_cast<const char *>(scratch) + proj_rowmap_offset(G));
     SGB_CUDA(cudaMemsetAsync(sino, 0, sizeof(float) * (size_t)G.na * G.nDet, st));
+    if (central_step(G) <= kDirectStep) {
+        int wb = 1;  // warps that share a row's groups
+        while (wb < kWarps && wb * kDirGroups * kDirGroup < G.nDet) wb *= 2;
+        const int z = (G.nDet + wb * kDirGroups * kDirGroup - 1) / (wb * kDirGroups * kDirGroup);
+        const size_t sd = project_direct_smem(G, wb);
+        const int blocks = split_items((G.nPix + kDirRows - 1) / kDirRows, (long long)G.na * z, resident(sd, 4));
+        const int rpc = blocks * kDirRows;
+        SGB_CUDA(cudaFuncSetAttribute(bdd_project_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sd));
+        bdd_project_direct_kernel<<<dim3(G.na, (G.nPix + rpc - 1) / rpc, z), kThreads, sd, st>>>(
+            G, info, detm, L, rmap, phantom, sino, rpc, wb);
+        return after_launch("bdd_project_direct_kernel");
+    }
     // rows split over CTAs so that each SM holds ~8 of them (views x row blocks)
     const int target = 8 * std::max(1, num_sms());
     int rsplit = std::max(1, std::min((G.nPix + kWarps - 1) / kWarps, (target + G.na - 1) / G.na));
@@ -681,15 +965,18 @@ int launch_bdd_project_main(const BddArgs &G, const float *phantom, float *sino,
 }
 
 int launch_bdd_back_setup(const BddArgs &G, void *scratch, cudaStream_t st) {
-    if (back_smem(G) > 220 * 1024) {
+    if (!back_fits(G)) {
         set_error("backproject_bdd: nPix=%d nDet=%d exceed the shared-memory tile", G.nPix, G.nDet);
         return SGB_ERR_ARG;
     }
     ViewInfo *info = static_cast<ViewInfo *>(scratch);
-    float4 *geo = reinterpret_cast<float4 *>(static_cast<char *>(scratch) + info_bytes(G.na)) + (size_t)G.na * (G.nDet + 1);
+    float *tab = reinterpret_cast<float *>(static_cast<char *>(scratch) + info_bytes(G.na));
+    float4 *geo = reinterpret_cast<float4 *>(static_cast<char *>(scratch) + back_geo_offset(G));
     bdd_setup_kernel<<<dim3(G.na, (G.nDet + kSetupChunk - 1) / kSetupChunk), kThreads, 0, st>>>(G, info, nullptr, nullptr,
                                                                                              geo);
     SGB_TRY(after_launch("bdd_setup_kernel"));
+    bdd_guess_kernel<<<G.na, kThreads, 0, st>>>(G, geo, tab);
+    SGB_TRY(after_launch("bdd_guess_kernel"));
     float4 *rmap = reinterpret_cast<float4 *>(static_cast<char *>(scratch) + back_rowmap_offset(G));
     const long long nr = (long long)G.na * G.nPix;
     bdd_rowmap_kernel<<<(unsigned)((nr + kThreads - 1) / kThreads), kThreads, 0, st>>>(G, info, rmap);
@@ -697,26 +984,28 @@ int launch_bdd_back_setup(const BddArgs &G, void *scratch, cudaStream_t st) {
 }
 
 int launch_bdd_back_main(const BddArgs &G, const float *sino, float *image, void *scratch, cudaStream_t st) {
-    const size_t smem = back_smem(G);
-    if (smem > 220 * 1024) {
+    if (!back_fits(G)) {
         set_error("backproject_bdd: nPix=%d nDet=%d exceed the shared-memory tile", G.nPix, G.nDet);
         return SGB_ERR_ARG;
     }
     const ViewInfo *info = static_cast<const ViewInfo *>(scratch);
-    float4 *tab = reinterpret_cast<float4 *>(static_cast<char *>(scratch) + info_bytes(G.na));
-    const float4 *geo = tab + (size_t)G.na * (G.nDet + 1);
+    float *tab = reinterpret_cast<float *>(static_cast<char *>(scratch) + info_bytes(G.na));
+    const float4 *geo = reinterpret_cast<const float4 *>(static_cast<const char *>(scratch) + back_geo_offset(G));
     const float4 *rmap = reinterpret_cast<const float4 *>(static_cast<const char *>(scratch) + back_rowmap_offset(G));
     SGB_CUDA(cudaMemsetAsync(image, 0, sizeof(float) * (size_t)G.nPix * G.nPix, st));
     bdd_fill_prefix_kernel<<<G.na, kThreads, 0, st>>>(G, sino, geo, tab);
     SGB_TRY(after_launch("bdd_fill_prefix_kernel"));
-    int gx = (G.nPix + kWarps - 1) / kWarps;
-    // views split over CTAs so that each SM holds ~8 of them (row blocks x view groups)
-    const int target = 8 * std::max(1, num_sms());
-    int vsplit = std::max(1, std::min(G.na, (target + gx - 1) / gx));
-    int vpc = (G.na + vsplit - 1) / vsplit;
-    vsplit = (G.na + vpc - 1) / vpc;
+    // a warp per (row, chunk of at most kBackGroups groups of 31 pixels)
+    const int ngroups = (G.nPix + 30) / 31, nchunk = (ngroups + kBackGroups - 1) / kBackGroups;
+    const int gpc = (ngroups + nchunk - 1) / nchunk;
+    const long long gx = ((long long)G.nPix * nchunk + kWarps - 1) / kWarps;
+    const size_t vbytes = sizeof(float) * (size_t)back_view_floats(G.nDet);
+    const int nstage = 2 * vbytes <= 220 * 1024 ? 2 : 1;
+    const size_t smem = nstage * vbytes;
+    const int vpc = split_items(G.na, gx, resident(smem, 5));
     SGB_CUDA(cudaFuncSetAttribute(bdd_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    bdd_back_kernel<<<dim3(gx, vsplit), kThreads, smem, st>>>(G, info, tab, rmap, image, vpc);
+    bdd_back_kernel<<<dim3((unsigned)gx, (G.na + vpc - 1) / vpc), kThreads, smem, st>>>(G, info, tab, rmap, image, vpc,
+                                                                                        nchunk, gpc, nstage);
     return after_launch("bdd_back_kernel");
 }
 
