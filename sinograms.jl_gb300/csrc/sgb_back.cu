@@ -233,37 +233,41 @@ ScanSlots scan_slots(int kind, int na, int nx, int ny, bool centred, bool source
 void back2_choose(Back2Args &A) {
     // Predicted time in us.  A view of a tile takes a thread its pixels' geometry and taps (instructions)
     // and the staging; a CTA's 8 warps issue 2.8 per clock between them when the SM has enough CTAs, and
-    // a CTA alone takes 2.2 times its share.  Starting, summing a split and interleaving take the rest.
-    const double geometry = A.mode == SGB_PAR ? 8 : (A.mode == SGB_FLAT ? 14 : 30);
+    // a CTA alone takes 2.4 times its share.  Starting, summing a split and interleaving take the rest.
+    // The constants were fitted to 600 launches of 32 scans (50^2 to 512^2, 60 to 1130 views, 1 to 12
+    // slices, every choice here); the choice takes 5 % more than the best of a scan's launches in the
+    // geometric mean, 26 % at most, where the timer's step was 10 %.
+    const double geometry = A.mode == SGB_PAR ? 4.4 : (A.mode == SGB_FLAT ? 6.3 : 13.5);
     const int sms = std::max(1, num_sms());
     Back2Args best = A;
     double best_us = 1e30;
-    for (int ns : {A.sym.ns, 1}) {
-        for (int sl : {1, 4}) {
-            if (sl == 4 && A.nslices == 1) continue;
-            const int p = ns * sl > 4 ? kB2P<4, 4> : kB2P<1, 1>, hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
-            const long long groups = floor_div_up(A.nslices, sl);
-            const long long tiles = (long long)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * p) * groups;
-            const double view = 0.0015 * (p * (geometry + ns * (sl == 1 ? 4 : 10)) + 12 + ns * A.w / 48.0);
-            for (int g = 1; g <= 8 && (g == 1 || A.nv >= 8 * g) && groups * g <= 65535; g++) {
-                const double busiest = (double)((tiles * g + sms - 1) / sms);
-                const int ctas = ns * sl == 1 ? kB2Ctas<1, 1> : kB2Ctas<4, 4>;
-                const int waves = (int)busiest / ctas, rest = (int)busiest % ctas;
-                const double share = waves * std::max(2.2, (double)ctas) + (rest ? std::max(2.2, (double)rest) : 0);
-                // a chunk of views takes at least its copies' latency
-                const int seg = ns * sl == 1 ? kB2Seg<1, 1> : kB2Seg<4, 4>;
-                const int views = floor_div_up(A.nv, g), vc = std::min({kB2V, seg / 2 / (ns * A.w * 4 * sl), views});
-                const double us = floor_div_up(views, vc) * std::max(vc * view * share, 0.9 * (waves + (rest ? 1 : 0))) + (g > 1 ? 1.5 + 0.1 * g : 0) +
-                                  (sl == 4 ? 3 + 8e-6 * A.nb * A.na * A.nslices / 6e3 : 0);
-                if (us < best_us) {
-                    best_us = us;
-                    best.sym.ns = ns;
-                    best.sl = sl;
-                    best.split = g;
-                    best.sym.hx = hx;
-                    best.sym.hy = hy;
-                    best.sym.turn = ns > 1 ? A.sym.turn : 0;
-                }
+    for (int form = 0; form < 3; form++) {  // slots; neither; slices in fours
+        const int ns = form == 0 ? A.sym.ns : 1, sl = form == 2 ? 4 : 1;
+        if (sl == 4 && A.nslices == 1) continue;
+        const int hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
+        const int ctas = ns * sl == 1 ? kB2Ctas<1, 1> : kB2Ctas<4, 1>, seg = ns * sl == 1 ? kB2Seg<1, 1> : kB2Seg<4, 1>;
+        const long long groups = floor_div_up(A.nslices, sl);
+        const long long tiles = (long long)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * kB2P) * groups;
+        const double tap = sl == 4 ? 6 : (ns > 1 ? 2.1 : 3.8);
+        const double view = 0.0015 * (kB2P * (geometry + ns * tap) + 10.8 + ns * A.w / 12.0);
+        for (int g = 1; g <= 8 && (g == 1 || A.nv >= 8 * g) && groups * g <= 65535; g++) {
+            if (g > 1 && tiles >= (long long)ctas * sms) break;  // the tiles alone fill the chip
+            const int busiest = (int)((tiles * g + sms - 1) / sms);
+            const int waves = busiest / ctas, rest = busiest % ctas;
+            const double share = waves * std::max(2.4, (double)ctas) + (rest ? std::max(2.4, (double)rest) : 0);
+            // a chunk of views takes at least its copies' latency
+            const int views = floor_div_up(A.nv, g), vc = std::max(1, std::min({kB2V, seg / 2 / (ns * A.w * 4 * sl), views}));
+            const double us = floor_div_up(views, vc) * std::max(vc * view * share, 0.9 * (waves + (rest ? 1 : 0))) +
+                              (g > 1 ? 1.5 + 0.1 * g + 0.3 * ns * sl * (double)(tiles * g) / sms : 0) +
+                              (sl == 4 ? 3 + 1e-5 * A.nb * (double)A.na * A.nslices : 0);
+            if (us < best_us) {
+                best_us = us;
+                best.sym.ns = ns;
+                best.sl = sl;
+                best.split = g;
+                best.sym.hx = hx;
+                best.sym.hy = hy;
+                best.sym.turn = ns > 1 ? A.sym.turn : 0;
             }
         }
     }

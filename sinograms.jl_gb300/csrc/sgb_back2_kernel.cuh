@@ -2,8 +2,7 @@
 // (src/fbp2/back-par.jl:206-315) and fbp_back_fan! / fbp_back_fan_xy (src/fbp2/back-fan.jl:215-336).
 // sgb_back2_<detector>.cu instantiate one detector each, so they compile in parallel.
 //
-// A CTA of 256 threads owns a tile of 32 x 32 pixels (32 x 16 with many sums per pixel): thread (tx, ty)
-// accumulates the pixels (tx, ty + 8k), which share the view's per-column terms and give
+// A CTA of 256 threads owns a tile of 32 x 32 pixels: thread (tx, ty) accumulates the pixels (tx, ty + 8k), which share the view's per-column terms and give
 // independent accumulation chains.  Views go in chunks.  For each view the CTA maps the
 // tile's four corners to detector bins: the parallel, flat and arc maps are monotone in the
 // angle under which the source sees a point, so over a rectangle in front of the source the
@@ -28,6 +27,13 @@
 //   NS  so do the images of a pixel under the scan's symmetry, each in its own view ("slots"): the
 //       quarter turns of a square image where 90 degrees are a whole number of views, else reflections
 //       in x and y (whose bins run the other way: staged reversed), else a half turn (scan_slots).
+// Not both: 16 sums per pixel halve the tile, and its segments' copies then cost what the geometry
+// saves (arc, 512^2 x 8 slices x 984 views: 798 to 1080 us by the view split; slices alone 744, slots
+// alone 929, neither 1908).  Slots alone: 320^2 x 673 parallel views 49 us against 50 to 66, 531 x 140
+// x 1130 arc views 95 against 132.
+//
+// Bound by issue (72 % of the slots in the stack above): per pixel and view the geometry, and per tap
+// one shared load and two multiply-adds.
 #pragma once
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
     const int W = A.w, VC = A.vc;                       // bins per segment, views per chunk
     const uint32_t SB = (uint32_t)(W * VB), BB = (uint32_t)(VC * NS) * SB;  // bytes per segment and per buffer
     constexpr int NA = NS * SL;               // accumulators per pixel
-    constexpr int P = kB2P<NS, SL>, T = kB2Y * P;  // passes and rows of a tile
+    constexpr int P = kB2P, T = kB2Y * P;  // passes and rows of a tile
     static_assert(P * NA * kB2X * kB2Y * 4 <= kB2Seg<NS, SL>, "the ranks' partial tiles reuse the segments");
     extern __shared__ __align__(16) unsigned char seg_s[];  // [2][VC][NS][W] staged bins
     __shared__ float4 par_s[2][kB2V];  // per view: sin, cos, form constants (bits), segment bound (bits)
@@ -423,7 +429,7 @@ int launch_slots(Back2Args A, cudaStream_t st) {
     SGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, seg));
     A.vc = std::min(kB2V, seg / 2 / (NS * A.w * 4 * SL));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(floor_div_up(A.sym.hx, kB2X), floor_div_up(A.sym.hy, kB2Y * kB2P<NS, SL>), groups * G);
+    cfg.gridDim = dim3(floor_div_up(A.sym.hx, kB2X), floor_div_up(A.sym.hy, kB2Y * kB2P), groups * G);
     cfg.blockDim = dim3(kB2X * kB2Y);
     cfg.dynamicSmemBytes = seg;
     cfg.stream = st;
@@ -444,8 +450,7 @@ int launch_slots(Back2Args A, cudaStream_t st) {
 
 template <int M>
 int launch(const Back2Args &A, cudaStream_t st) {
-    if (A.sl == 4)
-        return A.sym.ns == 4 ? launch_slots<M, 4, 4>(A, st) : (A.sym.ns == 2 ? launch_slots<M, 2, 4>(A, st) : launch_slots<M, 1, 4>(A, st));
+    if (A.sl == 4) return launch_slots<M, 1, 4>(A, st);
     return A.sym.ns == 4 ? launch_slots<M, 4, 1>(A, st) : (A.sym.ns == 2 ? launch_slots<M, 2, 1>(A, st) : launch_slots<M, 1, 1>(A, st));
 }
 

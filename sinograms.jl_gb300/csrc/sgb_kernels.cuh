@@ -144,10 +144,7 @@ struct Back2Args {
     ScanSlots sym;
 };
 constexpr int kB2X = 32, kB2Y = 8;  // pixels of a 2D tile that its 256 threads take at a time
-// such passes: rows of a tile / 8.  Two where a pixel has 16 sums, which leaves registers for a third
-// CTA per SM
-template <int NS, int SL>
-constexpr int kB2P = NS * SL > 4 ? 2 : 4;
+constexpr int kB2P = 4;             // such passes: rows of a tile / 8
 // CTAs that share an SM, by their registers and staged segments
 template <int NS, int SL>
 constexpr int kB2Ctas = NS * SL == 1 ? 5 : 3;
