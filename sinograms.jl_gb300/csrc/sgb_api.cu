@@ -124,14 +124,13 @@ int filter_status(int e) {
     return SGB_ERR_TIMEOUT;
 }
 
-// finish() plus, for synchronous calls, the filter's error word
+// Waits, for synchronous calls, and reads the filter's error word.
 // Plan calls keep their host staging buffers in the plan, so SGB_ASYNC also holds for host
 // pointers: the call returns with its copies and kernels enqueued (sgb_plan_sync reports).
 int plan_done(sgb_plan *P, int flags, cudaStream_t st) {
     if (flags & SGB_ASYNC) return SGB_OK;
-    SGB_TRY(finish(flags, st));
     int e = 0;
-    SGB_CUDA(cudaMemcpy(&e, P->filt_err, sizeof(int), cudaMemcpyDeviceToHost));
+    SGB_TRY(finish_read(&e, P->filt_err, sizeof e, st));
     return filter_status(e);
 }
 
@@ -680,9 +679,8 @@ int sgb_fdk(sgb_plan *P, const float *proj, float *image, int flags, void *strea
         if (!(flags & SGB_DEVICE_PTRS))
             SGB_CUDA(cudaMemcpyAsync(image, img_dev, nvox * sizeof(float), cudaMemcpyDeviceToHost, st));
         if (flags & SGB_ASYNC) return SGB_OK;
-        SGB_TRY(finish(flags, st));
         int err[2] = {0, 0};
-        SGB_CUDA(cudaMemcpy(err, P->flags.as<int>() + 2, sizeof err, cudaMemcpyDeviceToHost));
+        SGB_TRY(finish_read(err, P->flags.as<int>() + 2, sizeof err, st));
         if (err[0]) {
             set_error("fdk: back-projector reported error flags 0x%x (1: box undersized, 2/4: wait timeout)", err[0]);
             return (err[0] & 6) ? SGB_ERR_TIMEOUT : SGB_ERR_CUDA;
@@ -1341,9 +1339,8 @@ int sgb_batch_fdk_run(sgb_batch *B, int flags, void *stream) {
     SGB_CUDA(cudaGraphLaunch(B->exec, st));
     g_launches.fetch_add((long long)(B->plans.size() + B->classes.size()), std::memory_order_relaxed);
     if (flags & SGB_ASYNC) return SGB_OK;
-    SGB_CUDA(cudaStreamSynchronize(st));
     int err[2] = {0, 0};
-    SGB_CUDA(cudaMemcpy(err, B->flags.p, sizeof err, cudaMemcpyDeviceToHost));
+    SGB_TRY(finish_read(err, B->flags.p, sizeof err, st));
     if (err[0]) {
         set_error("batch_fdk: back-projector reported error flags 0x%x (1: box undersized, 2/4: wait timeout)",
                   err[0]);

