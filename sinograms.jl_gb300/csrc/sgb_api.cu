@@ -720,6 +720,20 @@ int sgb_fdk(sgb_plan *P, const float *proj, float *image, int flags, void *strea
     return plan_done(P, flags, st);
 }
 
+// Room for n bytes in a workspace that the call can do without: not grown while the stream is being
+// captured, nor past the device's memory.
+static bool grow_between_captures(DevBuf &b, size_t n, cudaStream_t st) {
+    if (b.p && n <= b.bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    if (b.reserve(n) == SGB_OK) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Back-projection of a 2D plan's filtered slices.
 static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices, cudaStream_t st) {
     const sgb_sino_geom &g = P->sg;
@@ -745,12 +759,17 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
     A.sino = sino;
     A.image = image;
     A.nslices = nslices;
-    back2_choose(A);
+    const Back2Args all = A;
+    back2_choose(A, true);
     if (A.sl == 4) {
         const long long n = (long long)g.nb * g.na;
-        SGB_TRY(P->inter.reserve(sizeof(float) * 4 * n * floor_div_up(nslices, 4)));
-        SGB_TRY(launch_interleave4(sino, P->inter.as<float>(), n, nslices, st));
-        A.sino4 = P->inter.as<float>();
+        if (grow_between_captures(P->inter, sizeof(float) * 4 * n * floor_div_up(nslices, 4), st)) {
+            SGB_TRY(launch_interleave4(sino, P->inter.as<float>(), n, nslices, st));
+            A.sino4 = P->inter.as<float>();
+        } else {  // slice by slice
+            A = all;
+            back2_choose(A, false);
+        }
     }
     return launch_back2(A, st);
 }
@@ -964,7 +983,7 @@ static int back2_seam(float *image, const float *sino, int nb, int na, const dou
     A.sym = ScanSlots{1, nx, ny, 0, 0, {{0, 1, 0, 0}}};
     // the axes are the caller's, spaced as they like: their mean spacing
     back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0);
-    back2_choose(A);
+    back2_choose(A, false);
     SGB_TRY(launch_back2(A, st));
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(image, img_dev, sizeof(float) * (size_t)nx * ny, cudaMemcpyDeviceToHost, st));

@@ -230,7 +230,7 @@ ScanSlots scan_slots(int kind, int na, int nx, int ny, bool centred, bool source
     return S;
 }
 
-void back2_choose(Back2Args &A) {
+void back2_choose(Back2Args &A, bool fours) {
     // Predicted time in us.  A view of a tile takes a thread its pixels' geometry and taps (instructions)
     // and the staging; a CTA's 8 warps issue 2.8 per clock between them when the SM has enough CTAs, and
     // a CTA alone takes 2.4 times its share.  Starting, summing a split and interleaving take the rest.
@@ -243,7 +243,7 @@ void back2_choose(Back2Args &A) {
     double best_us = 1e30;
     for (int form = 0; form < 3; form++) {  // slots; neither; slices in fours
         const int ns = form == 0 ? A.sym.ns : 1, sl = form == 2 ? 4 : 1;
-        if (sl == 4 && A.nslices == 1) continue;
+        if (sl == 4 && (A.nslices == 1 || !fours)) continue;
         const int hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
         const int ctas = ns * sl == 1 ? kB2Ctas<1, 1> : kB2Ctas<4, 1>, seg = ns * sl == 1 ? kB2Seg<1, 1> : kB2Seg<4, 1>;
         const long long groups = floor_div_up(A.nslices, sl);

@@ -32,7 +32,8 @@
 // alone 929, neither 1908).  Slots alone: 320^2 x 673 parallel views 49 us against 50 to 66, 531 x 140
 // x 1130 arc views 95 against 132.
 //
-// Bound by issue (72 % of the slots in the stack above): per pixel and view the geometry, and per tap
+// The stack above is bound by its 16-byte shared loads (75 % of the wavefronts, issue 60 %), four
+// wavefronts a tap; single images by issue (70 to 79 %): per pixel and view the geometry, and per tap
 // one shared load and two multiply-adds.
 #pragma once
 #include <cooperative_groups.h>

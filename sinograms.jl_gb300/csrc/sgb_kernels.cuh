@@ -156,8 +156,8 @@ constexpr int kB2Seg = (NS * SL == 1 ? 40 : 64) * 1024;
 // sets w
 void back2_window(Back2Args &A, double dx, double dy);
 // The launch predicted to be the fastest: with or without the slots, slices one by one or in fours, and
-// the view split.
-void back2_choose(Back2Args &A);
+// the view split.  `fours`: the caller has room for the interleaved slices.
+void back2_choose(Back2Args &A, bool fours);
 int launch_back2(const Back2Args &A, cudaStream_t st);
 // (n, nslices) -> (4, n, ceil(nslices / 4)); the last group's missing slices are zeros
 int launch_interleave4(const float *in, float *out, long long n, int nslices, cudaStream_t st);
