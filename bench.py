@@ -101,14 +101,14 @@ def _issue_roofline(updates, back_ms, clocks, form):
     instructions per update come from the committed ncu capture of this kernel (storage form
     `form`) at this size; the peak is 152 SMs x 4 schedulers x 32 lanes per cycle at the sampled
     SM clock."""
-    ipu = _from_profile("fdk_tma_kernel_bench_issue.md", f"thread_instructions_per_update_{form}")
+    ipu = _from_profile("fdk_mirror_kernel_bench_issue.md", f"thread_instructions_per_update_{form}")
     mhz = (clocks or {}).get("sm_mhz") or 2070.0
     peak = 152 * 4 * 32 * mhz * 1e6
     if ipu is None:
         return None
     achieved = ipu * updates / (back_ms / 1e3)
     return {"thread_instructions_per_update": ipu, "achieved_per_s": achieved, "peak_per_s": peak,
-            "frac": achieved / peak, "source": "profiles/fdk_tma_kernel_bench_issue.md (ncu smsp__inst_executed)"}
+            "frac": achieved / peak, "source": "profiles/fdk_mirror_kernel_bench_issue.md (ncu smsp__inst_executed)"}
 
 
 def _bp_roofline(updates, back_ms):
@@ -357,10 +357,10 @@ def run_ours(args):
                                   "ms_per_step": e2e_1s * 1e3 / args.steps,
                                   "pipeline": "fdk(plan, host proj, out=host volume) on one plan and one stream, "
                                               "synchronous: copies in, filter, back-projection, copy out"}},
-        "roofline": {"bound": "hbm", "kernel": "fdk_tma_kernel", "achieved": achieved, "peak": hbm,
+        "roofline": {"bound": "hbm", "kernel": "fdk_mirror_kernel", "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_source": hbm_src,
                      "alg_bytes_per_launch": alg_bytes,
-                     "traffic": _from_profile("fdk_tma_kernel_bench_dram.md", f"traffic_bytes_per_launch_{head}"),
+                     "traffic": _from_profile("fdk_mirror_kernel_bench_dram.md", f"traffic_bytes_per_launch_{head}"),
                      "issue": _issue_roofline(upd, f["back_ms"], f["clocks"], head),
                      "fp32_issue": {"flops_per_update": F_UPD,
                                     "achieved_tflops": F_UPD * upd / (f["back_ms"] / 1e3) / 1e12,
