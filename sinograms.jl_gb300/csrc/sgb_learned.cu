@@ -16,7 +16,7 @@
 //   conv_fwd_c1   the same for one output channel
 //   conv_wgrad    dW[co,ci,k] = sum_{r,t} g[r,co,t] x[r,ci,t+k-4], db[co] = sum g, SIMT, for the
 //                 1 -> 32 and 32 -> 1 layers
-//   gelu_bwd, loss (MSE on the residual), adam
+//   loss (MSE on the residual), adam
 // Activations are (rows, channels, L) with L = detector samples, zero padded by 4.
 //
 // Inference (sgb_lf_apply) runs the whole network in one persistent kernel, lf_tc_fused,
@@ -74,7 +74,10 @@ constexpr int kCoPer = 4, kTPer = 8;
 
 // y[r, co, t] for kT positions of one row: thread (cg, tg) computes channels 4 cg .. 4 cg + 3 at
 // positions t0 + tg + 16 i (i < 8), so the 16 lanes of a channel store 16 consecutive positions.
-// With ACT it stores GELU(y) and, for the backward pass, GELU'(y).
+// With ACT it stores GELU(y) and, for the backward pass, GELU'(y); without, in the backward pass, it
+// takes the gradient y through the GELU below: y * dg.  A pass of its own for that product read and
+// wrote the 32 channels once more (4096 x 888: 104 + 260 us, now 175: 930 MB at 5.3 TB/s); with dg
+// loaded only after the sums it took 307.
 template <int CIN, int COUT, bool ACT, bool BIAS>
 __global__ void __launch_bounds__(128) conv_fwd(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
                                                 const float *__restrict__ b, float *__restrict__ dg,
@@ -87,6 +90,18 @@ __global__ void __launch_bounds__(128) conv_fwd(const float *__restrict__ in, co
     const long long r = blockIdx.y;
     const int t0 = blockIdx.x * kT;
     const float *x = in + r * CIN * (long long)L;
+    const int cg = threadIdx.x / kLanes, tg = threadIdx.x % kLanes;
+    const int co0 = cg * kCoPer;
+    float dv[kCoPer][kTPer];  // on their way while the inputs are staged and summed
+    if (!ACT) {
+#pragma unroll
+        for (int j = 0; j < kCoPer; j++)
+#pragma unroll
+            for (int i = 0; i < kTPer; i++) {
+                const int t = t0 + tg + kLanes * i;
+                dv[j][i] = t < L ? __ldcs(dg + (r * COUT + co0 + j) * (long long)L + t) : 0.f;
+            }
+    }
     for (int i = threadIdx.x; i < CIN * (kT + 2 * kPad); i += 128) {
         const int ci = i / (kT + 2 * kPad), j = i % (kT + 2 * kPad);
         const int t = t0 + j - kPad;
@@ -94,8 +109,6 @@ __global__ void __launch_bounds__(128) conv_fwd(const float *__restrict__ in, co
     }
     for (int i = threadIdx.x; i < COUT * CIN * kK; i += 128) ws[i] = __bfloat162float(W[i]);
     __syncthreads();
-    const int cg = threadIdx.x / kLanes, tg = threadIdx.x % kLanes;
-    const int co0 = cg * kCoPer;
     float acc[kCoPer][kTPer];
 #pragma unroll
     for (int j = 0; j < kCoPer; j++)
@@ -128,44 +141,97 @@ __global__ void __launch_bounds__(128) conv_fwd(const float *__restrict__ in, co
                 dg[o] = d;
                 out[o] = g;
             } else {
-                out[o] = acc[j][i];
+                out[o] = acc[j][i] * dv[j][i];
             }
         }
 }
 
-// one output channel (the last layer): a thread per position, the CTA's CIN x (128 + 8) inputs
-// staged in shared memory first
-template <int CIN>
+// One output channel (the last layer).  A thread has four neighbouring positions, whose 12 inputs of a
+// channel are three 16-byte shared loads for 36 FMAs; the channels arrive in four groups by cp.async,
+// and a group is summed while the later ones are in flight.  Bound by DRAM (the 32 channels read once):
+// 4096 x 888, 113 us, 4.1 TB/s.  With a position per thread each FMA took a shared load of its input and
+// one of its weight, 272 us.  Sums run over channel and tap in the same order for every split.
+constexpr int kC1Pos = 4;                // positions per thread
+constexpr int kC1Tile = 128 * kC1Pos;   // positions per CTA, at most
+constexpr int kC1Groups = 4;
+
+__device__ __forceinline__ void cp_async_zfill(float *dst, const float *src, bool in, int bytes) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (bytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
+// blockDim = tile / kC1Pos threads; V: floats per copy (4 where rows start on 16 bytes, else 1)
+template <int CIN, int V>
 __global__ void __launch_bounds__(128) conv_fwd_c1(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
-                                                   const float *__restrict__ b, float *__restrict__ out, int L,
-                                                   bool bias) {
-    __shared__ float ws[CIN * kK];
-    __shared__ float xs[CIN][128 + 2 * kPad];
-    for (int i = threadIdx.x; i < CIN * kK; i += blockDim.x) ws[i] = __bfloat162float(W[i]);
+                                                   const float *__restrict__ b, float *__restrict__ out, int L) {
+    static_assert(CIN % kC1Groups == 0 && kPad == 4 && kK == 9, "three float4 per thread and channel");
+    extern __shared__ __align__(16) float sm[];
+    float *ws = sm;                  // [CIN][12]
+    float *xs = ws + CIN * 12;       // [CIN][tile + 8]
+    const int tile = blockDim.x * kC1Pos, row = tile + 2 * kPad;
     const long long r = blockIdx.y;
-    const int t0 = blockIdx.x * 128;
+    const int t0 = blockIdx.x * tile;
     const float *x = in + r * CIN * (long long)L;
-    // eight loads in flight per thread before their stores
-    constexpr int kRow = 128 + 2 * kPad, kTot = CIN * kRow;
-    for (int i0 = threadIdx.x; i0 < kTot; i0 += 8 * 128) {
-        float v[8];
+    constexpr int kPer = CIN / kC1Groups;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int i = i0 + u * 128, t = t0 + i % kRow - kPad;
-            v[u] = (i < kTot && t >= 0 && t < L) ? x[(long long)(i / kRow) * L + t] : 0.f;
+    for (int g = 0; g < kC1Groups; g++) {
+        for (int c = g * kPer, j = threadIdx.x * V; c < (g + 1) * kPer;) {
+            const int t = t0 + j - kPad;
+            const bool ok = t >= 0 && t < L;  // V = 4: L and t are multiples of 4, all four or none
+            cp_async_zfill(xs + c * row + j, ok ? x + (long long)c * L + t : x, ok, V * 4);
+            j += blockDim.x * V;
+            if (j >= row) {
+                j -= row;
+                c++;
+            }
         }
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (i0 + u * 128 < kTot) xs[(i0 + u * 128) / kRow][(i0 + u * 128) % kRow] = v[u];
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    __syncthreads();
-    const int t = t0 + threadIdx.x;
-    if (t >= L) return;
-    float acc = bias ? b[0] : 0.f;
-    for (int ci = 0; ci < CIN; ci++)
+    for (int i = threadIdx.x; i < CIN * kK; i += blockDim.x) ws[i / kK * 12 + i % kK] = __bfloat162float(W[i]);
+    float acc[kC1Pos];
 #pragma unroll
-        for (int k = 0; k < kK; k++) acc = fmaf(ws[ci * kK + k], xs[ci][threadIdx.x + k], acc);
-    out[r * (long long)L + t] = acc;
+    for (int i = 0; i < kC1Pos; i++) acc[i] = b[0];
+#pragma unroll
+    for (int g = 0; g < kC1Groups; g++) {
+        if (g == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (g == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (g == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+#pragma unroll 2
+        for (int c = g * kPer; c < (g + 1) * kPer; c++) {
+            const float4 *xp = reinterpret_cast<const float4 *>(xs + c * row) + threadIdx.x;
+            const float4 *wp = reinterpret_cast<const float4 *>(ws + c * 12);
+            const float4 x0 = xp[0], x1 = xp[1], x2 = xp[2], w0 = wp[0], w1 = wp[1];
+            const float v[12] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, x2.x, x2.y, x2.z, x2.w};
+            const float w[kK] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, ws[c * 12 + 8]};
+#pragma unroll
+            for (int k = 0; k < kK; k++)
+#pragma unroll
+                for (int i = 0; i < kC1Pos; i++) acc[i] = fmaf(w[k], v[i + k], acc[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kC1Pos; i++) {
+        const int t = t0 + threadIdx.x * kC1Pos + i;
+        if (t < L) out[r * (long long)L + t] = acc[i];
+    }
+}
+
+template <int CIN>
+int launch_conv_c1(const float *in, const __nv_bfloat16 *W, const float *b, float *out, int L, long long R,
+                   cudaStream_t st) {
+    // the fewest tiles of at most kC1Tile, of equal whole warps
+    const int n = (L + kC1Tile - 1) / kC1Tile, warp = 32 * kC1Pos, threads = (L + n * warp - 1) / (n * warp) * 32;
+    const size_t smem = sizeof(float) * CIN * (12 + threads * kC1Pos + 2 * kPad);
+    const bool vec = L % 4 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
+    auto k = vec ? conv_fwd_c1<CIN, 4> : conv_fwd_c1<CIN, 1>;
+    SGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<dim3(n, (unsigned)R), threads, smem, st>>>(in, W, b, out, L);
+    return after_launch("conv_fwd_c1");
 }
 
 // -------------------------------------------------------------- weight grad
@@ -276,12 +342,6 @@ __global__ void __launch_bounds__(256) conv_wgrad(const float *__restrict__ in, 
 }
 
 // ------------------------------------------------------------- elementwise
-// through a GELU in the backward pass: g *= GELU'(pre), the derivative stored by the forward
-__global__ void gelu_bwd(float *__restrict__ g, const float *__restrict__ dg, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        g[i] *= dg[i];
-}
-
 // residual MSE: net output o, input z, target y (all (R, L)); loss = mean((z + s o - y)^2)/s^2
 // in normalised units; grad wrt o = 2 (o - (y - z)/s) / N.
 __global__ void mse_residual(const float *__restrict__ o, const float *__restrict__ z, const float *__restrict__ y,
@@ -1309,10 +1369,8 @@ int lf_forward(sgb_lf *F, long long R, int L, cudaStream_t st) {
     for (int l = 1; l < kLayers - 1; l++)
         SGB_TRY((launch_conv32_tc<true, true>(F, F->act[l].as<float>(), l - 1, p + F->off.b[l], F->dgl[l].as<float>(),
                                               F->act[l + 1].as<float>(), L, R, st)));
-    conv_fwd_c1<kC><<<dim3((L + 127) / 128, (unsigned)R), 128, 0, st>>>(
-        F->act[kLayers - 1].as<float>(), wb + F->wbase[kLayers - 1], p + F->off.b[kLayers - 1],
-        F->act[kLayers].as<float>(), L, true);
-    return after_launch("conv_fwd_c1");
+    return launch_conv_c1<kC>(F->act[kLayers - 1].as<float>(), wb + F->wbase[kLayers - 1], p + F->off.b[kLayers - 1],
+                              F->act[kLayers].as<float>(), L, R, st);
 }
 
 int lf_tc_workspace(sgb_lf *F) {
@@ -1362,14 +1420,10 @@ int lf_backward(sgb_lf *F, long long R, int L, cudaStream_t st) {
     conv_wgrad<kC, 1><<<wgrid, 256, 0, st>>>(F->act[4].as<float>(), F->gz.as<float>(), g + F->off.w[4],
                                              g + F->off.b[4], L, R);
     SGB_TRY(after_launch("conv_wgrad"));
-    SGB_TRY((launch_conv<1, kC, false, false>(F->gz.as<float>(), wt + F->wbase[4], nullptr, nullptr,
-                                              F->ga.as<float>(), L, R, st)));
+    // every data-gradient pass takes the gradient through the GELU of the layer beneath in its epilogue
+    SGB_TRY((launch_conv<1, kC, false, false>(F->gz.as<float>(), wt + F->wbase[4], nullptr,
+                                              F->dgl[kLayers - 2].as<float>(), F->ga.as<float>(), L, R, st)));
     float *gcur = F->ga.as<float>(), *gnext = F->gb.as<float>();
-    // through GELU of layer 3; the data-gradient passes below take the gradient through the
-    // GELU of the layer beneath in their epilogue
-    gelu_bwd<<<grid_for(R * kC * (long long)L), 256, 0, st>>>(gcur, F->dgl[kLayers - 2].as<float>(),
-                                                              R * kC * (long long)L);
-    SGB_TRY(after_launch("gelu_bwd"));
     for (int l = kLayers - 2; l >= 1; l--) {
         SGB_TRY(launch_wgrad32_tc(F, F->act[l].as<float>(), gcur, g + F->off.w[l], g + F->off.b[l], L, R, st));
         SGB_TRY((launch_conv32_tc<false, false>(F, gcur, l + 2, nullptr, F->dgl[l - 1].as<float>(), gnext, L, R, st)));
