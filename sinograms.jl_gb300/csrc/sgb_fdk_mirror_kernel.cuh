@@ -396,8 +396,11 @@ __device__ __forceinline__ void mir_fill(const FdkMirrorArgs &M, const CUtensorM
         S.fhi = (float)(hi + 1) - kSlack;
         S.t0 = t0;
         S.zoff = (uint32_t)A.box_bytes + (uint32_t)((2 * t0 + A.H + 1) * A.W * 8);
-        mbar_arrive_expect_tx(full, (uint32_t)(NS * A.W * A.H * 8));
     }
+    // lane 1's columns too have to be in the stage before lane 0's arrival, which publishes it: shuffles
+    // order no memory
+    __syncwarp();
+    if (lane == 0) mbar_arrive_expect_tx(full, (uint32_t)(NS * A.W * A.H * 8));
     __syncwarp();
     if (lane < NS)
         tma_load_3d(dst + (size_t)lane * A.box_bytes, map, s0 * 2, z ? M.m2 - t0 - A.H - 1 : t0, view, full);
