@@ -301,6 +301,14 @@ SGB_API int sgb_plan_info(const sgb_plan *plan, int *info, int n);
 /* Overrides the autotuner's choice of how many launches an FDK plan splits its views over (the
  * later launches add to the volume); 1 <= passes <= min(8, na).  Results agree to rounding. */
 SGB_API int sgb_plan_set_view_passes(sgb_plan *plan, int passes);
+/* Launch of a 2D plan's back-projection (no counterpart in the reference).  set_back_form overrides the
+ * plan's choice: form 0 takes a pixel at a time, 1 each pixel together with its images under the scan's
+ * symmetry (those that have one), 2 four slices at a time, -1 leaves it to the plan; `split` (1..8, 0: the
+ * plan's choice) thread blocks share a tile's views.  back_form reports the launch for nslices slices:
+ * info[0] = images per pixel (1, 2 or 4), info[1] = slices at a time (1 or 4), info[2] = split.  Results
+ * agree to rounding. */
+SGB_API int sgb_plan_set_back_form(sgb_plan *plan, int form, int split);
+SGB_API int sgb_plan_back_form(const sgb_plan *plan, int nslices, int *info, int n);
 /* On-chip peaks the back-projectors' roofline is stated against (no reference counterpart),
  * measured on `stream` with CUDA events: peaks[0] = shared-memory load bandwidth (bytes/s,
  * conflict-free 16-byte loads), peaks[1] = FP32 FMA throughput (flop/s, an FMA counting 2). */

@@ -93,6 +93,7 @@ struct sgb_plan {
     // staging for host-pointer calls
     DevBuf in_buf, filt_buf, img_buf;
     DevBuf inter;  // 2D stacks: the filtered slices interleaved in fours
+    int want_form = B2_FORM_AUTO, want_split = 0;  // the 2D launch that the caller asked for
     // F16 form: the filter's FP32 rows before they become FP16 quads, and the device words
     // (max |y| as bits, inverse scale) of the quads' power-of-two scale
     DevBuf qtmp, qword;
@@ -734,8 +735,8 @@ static bool grow_between_captures(DevBuf &b, size_t n, cudaStream_t st) {
     return false;
 }
 
-// Back-projection of a 2D plan's filtered slices.
-static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices, cudaStream_t st) {
+// A 2D plan's back-projection of nslices, but for the launch's choice and the buffers.
+static Back2Args back2_args(const sgb_plan *P, int nslices) {
     const sgb_sino_geom &g = P->sg;
     Back2Args A{};
     A.mask = P->mask_dev;
@@ -756,9 +757,18 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
     back2_window(A, P->deltas[0] / g.d, P->deltas[1] / g.d);
     A.sym = scan_slots(g.kind, g.na, P->nx, P->ny, 2.0 * A.wb == g.nb + 1.0, g.source_offset == 0, g.orbit, g.orbit_start,
                        P->deltas, P->offsets, true);
+    A.nslices = nslices;
+    A.want_form = P->want_form;
+    A.want_split = P->want_split;
+    return A;
+}
+
+// Back-projection of a 2D plan's filtered slices.
+static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices, cudaStream_t st) {
+    const sgb_sino_geom &g = P->sg;
+    Back2Args A = back2_args(P, nslices);
     A.sino = sino;
     A.image = image;
-    A.nslices = nslices;
     const Back2Args all = A;
     back2_choose(A, true);
     if (A.sl == 4) {
@@ -772,6 +782,26 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
         }
     }
     return launch_back2(A, st);
+}
+
+int sgb_plan_set_back_form(sgb_plan *P, int form, int split) {
+    SGB_REQUIRE(P && !P->ct, "plan_set_back_form: needs a 2D plan");
+    SGB_REQUIRE(form >= B2_FORM_AUTO && form <= B2_FORM_FOURS, "plan_set_back_form: unknown form %d", form);
+    SGB_REQUIRE(split >= 0 && split <= 8, "plan_set_back_form: split must be in [0, 8], got %d", split);
+    P->want_form = form;
+    P->want_split = split;
+    return SGB_OK;
+}
+
+int sgb_plan_back_form(const sgb_plan *P, int nslices, int *info, int n) {
+    SGB_REQUIRE(P && !P->ct && info && n >= 3, "plan_back_form: needs a 2D plan and room for 3 values");
+    SGB_REQUIRE(nslices >= 1 && nslices <= 65535, "plan_back_form: nslices must be in [1, 65535]");
+    Back2Args A = back2_args(P, nslices);
+    back2_choose(A, true);
+    info[0] = A.sym.ns;
+    info[1] = A.sl;
+    info[2] = A.split;
+    return SGB_OK;
 }
 
 int sgb_fbp(sgb_plan *P, const float *sino, float *image, int nslices, int flags, void *stream) {
@@ -981,6 +1011,7 @@ static int back2_seam(float *image, const float *sino, int nb, int na, const dou
     A.dso_ds = (float)(dso / ds);
     A.so_ds = (float)(source_offset / ds);
     A.sym = ScanSlots{1, nx, ny, 0, 0, {{0, 1, 0, 0}}};
+    A.want_form = B2_FORM_AUTO;
     // the axes are the caller's, spaced as they like: their mean spacing
     back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0);
     back2_choose(A, false);

@@ -241,17 +241,20 @@ void back2_choose(Back2Args &A, bool fours) {
     const int sms = std::max(1, num_sms());
     Back2Args best = A;
     double best_us = 1e30;
-    for (int form = 0; form < 3; form++) {  // slots; neither; slices in fours
-        const int ns = form == 0 ? A.sym.ns : 1, sl = form == 2 ? 4 : 1;
-        if (sl == 4 && (A.nslices == 1 || !fours)) continue;
+    for (int form : {B2_FORM_SLOTS, B2_FORM_PLAIN, B2_FORM_FOURS}) {
+        const int ns = form == B2_FORM_SLOTS ? A.sym.ns : 1, sl = form == B2_FORM_FOURS ? 4 : 1;
+        if (A.want_form != B2_FORM_AUTO && form != A.want_form && !(A.want_form == B2_FORM_FOURS && !fours)) continue;
+        if (sl == 4 && (!fours || (A.nslices == 1 && A.want_form != B2_FORM_FOURS))) continue;
         const int hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
         const int ctas = ns * sl == 1 ? kB2Ctas<1, 1> : kB2Ctas<4, 1>, seg = ns * sl == 1 ? kB2Seg<1, 1> : kB2Seg<4, 1>;
         const long long groups = floor_div_up(A.nslices, sl);
         const long long tiles = (long long)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * kB2P) * groups;
         const double tap = sl == 4 ? 6 : (ns > 1 ? 2.1 : 3.8);
         const double view = 0.0015 * (kB2P * (geometry + ns * tap) + 10.8 + ns * A.w / 12.0);
-        for (int g = 1; g <= 8 && (g == 1 || A.nv >= 8 * g) && groups * g <= 65535; g++) {
-            if (g > 1 && tiles >= (long long)ctas * sms) break;  // the tiles alone fill the chip
+        for (int g = 1; g <= 8 && groups * g <= 65535; g++) {
+            if (A.want_split ? g != A.want_split
+                             // eight views a rank at least; and the tiles alone may fill the chip
+                             : g > 1 && (A.nv < 8 * g || tiles >= (long long)ctas * sms)) continue;
             const int busiest = (int)((tiles * g + sms - 1) / sms);
             const int waves = busiest / ctas, rest = busiest % ctas;
             const double share = waves * std::max(2.4, (double)ctas) + (rest ? std::max(2.4, (double)rest) : 0);

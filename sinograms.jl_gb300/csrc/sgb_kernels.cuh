@@ -142,7 +142,10 @@ struct Back2Args {
     int sl, split;  // slices per CTA (1 or 4) and CTAs that share a tile's views (back2_choose)
     int w, vc;  // staged bins per segment (<= 256; longer ones read global memory) and views per chunk
     ScanSlots sym;
+    int want_form, want_split;  // the launch asked for: B2_FORM_AUTO and 0 leave the choice to back2_choose
 };
+// Forms of a 2D launch: a pixel at a time; with its images under the scan's symmetry; for four slices.
+enum { B2_FORM_AUTO = -1, B2_FORM_PLAIN = 0, B2_FORM_SLOTS = 1, B2_FORM_FOURS = 2 };
 constexpr int kB2X = 32, kB2Y = 8;  // pixels of a 2D tile that its 256 threads take at a time
 constexpr int kB2P = 4;             // such passes: rows of a tile / 8
 // CTAs that share an SM, by their registers and staged segments

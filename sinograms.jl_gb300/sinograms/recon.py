@@ -104,6 +104,18 @@ class FBPNormalPlan(_Plan):
     def view_weight(self):
         return fbp_view_weight(self.rg)
 
+    def set_back_form(self, form: str = "auto", split: int = 0):
+        """Override the back-projection's launch: "plain", "symmetric" (pixels together with their images
+        under the scan's symmetry) or "fours" (four slices at a time); `split` blocks share a tile's views."""
+        _status(_lib.lib().sgb_plan_set_back_form(self._h, ("auto", "plain", "symmetric", "fours").index(form) - 1,
+                                                  int(split)), "plan_set_back_form")
+
+    def back_form(self, nslices: int = 1) -> dict:
+        """The back-projection's launch for a stack of `nslices`."""
+        a = np.zeros(3, dtype=np.int32)
+        _status(_lib.lib().sgb_plan_back_form(self._h, int(nslices), ptr(a), 3), "plan_back_form")
+        return dict(images=int(a[0]), slices=int(a[1]), split=int(a[2]))
+
 
 class FDKplan(_Plan):
     """FDKplan (plan3.jl:13-23): rg, ig, filter (Hk), view_weight."""
