@@ -157,6 +157,19 @@ __device__ __forceinline__ void b2_tap(uint32_t a, float wa, float wb, float (&a
     }
 }
 
+// Taps at the detector's ends.  The reference takes 1 <= bb < nb (back-par.jl:307, back-fan.jl:328); a slot
+// whose bins run the other way sees nb + 1 - bb, and so takes 1 < bb <= nb.  At bb == 1 (`first`) only the
+// slots that run along take the tap; at bb == nb (`last`) only the reversed ones, with the weight on bin nb,
+// the far one of the two before it.  Parallel views along an axis put whole pixel columns exactly there.
+struct B2End {
+    bool first, last;
+};
+template <int NS>
+__device__ __forceinline__ B2End b2_end(float bb, int nb) {
+    if constexpr (NS == 1) return {false, false};
+    return {bb == 1.f, bb == (float)nb};
+}
+
 __device__ __forceinline__ void b2_copy4(uint32_t dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -345,10 +358,21 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
                 // segment, so j < jlim is the reference's tap rule (back-par.jl:307,
                 // back-fan.jl:328) for this tile.
                 const float m = __fadd_rd(bb, kMagic);
-                const uint32_t e = __float_as_uint(m) - jbias;
+                const B2End end = b2_end<NS>(bb, A.nb);
+                const uint32_t e = __float_as_uint(m) - jbias - end.last;
                 const bool ok = e < jlim && in;
-                const float wb = ok ? w2 * (bb - (m - kMagic)) : 0.f, wa = ok ? w2 - wb : 0.f;
+                const float f = end.last ? 1.f : bb - (m - kMagic);
+                const float wb = ok ? w2 * f : 0.f, wa = ok ? w2 - wb : 0.f;
                 const uint32_t ad = seg + (uint32_t)VB * (ok ? e : (uint32_t)(W - 2));
+                if (NS > 1 && (end.first || end.last)) {
+#pragma unroll
+                    for (int j = 0; j < NS; j++) {
+                        bool rev;
+                        slot_view(A.sym, A.na, j, va + c * VC + vi, &rev);
+                        if (rev == end.last) b2_tap<SL>(ad + (uint32_t)j * SB, wa, wb, acc[k][j]);
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int j = 0; j < NS; j++) b2_tap<SL>(ad + (uint32_t)j * SB, wa, wb, acc[k][j]);
             }
@@ -364,13 +388,15 @@ __global__ void __launch_bounds__(kB2X *kB2Y, (kB2Ctas<NS, SL>))
                 bool fr, in;
                 const float bb = b2_pix<M>(A, a, b, y[k], p.x, p.y, &w2, &fr, &in);
                 const float m = __fadd_rd(bb, kMagic);
-                const uint32_t il1 = __float_as_uint(m) - 0x4B400001u;  // floor(bb) - 1
+                const B2End end = b2_end<NS>(bb, A.nb);
+                const uint32_t il1 = __float_as_uint(m) - 0x4B400001u - end.last;  // floor(bb) - 1
                 if (in && il1 < nbm1) {
-                    const float wb = w2 * (bb - (m - kMagic)), wa = w2 - wb;
+                    const float wb = w2 * (end.last ? 1.f : bb - (m - kMagic)), wa = w2 - wb;
 #pragma unroll
                     for (int j = 0; j < NS; j++) {
                         bool rev = false;
                         const int row = NS == 1 ? v : slot_view(A.sym, A.na, j, v, &rev);
+                        if (NS > 1 && (rev ? end.first : end.last)) continue;
                         const long long o = row * vstride + (rev ? nbm1 - il1 : il1);
                         const int step = rev ? -1 : 1;
                         if constexpr (SL == 4) {
