@@ -92,7 +92,9 @@ struct sgb_plan {
     float scale = 1.f;
     // staging for host-pointer calls
     DevBuf in_buf, filt_buf, img_buf;
-    DevBuf inter;  // 2D stacks: the filtered slices interleaved in fours
+    // 2D stacks: where a call's interleaved slices come from (stack_buffer)
+    cudaMemPool_t stacks = nullptr;
+    std::mutex stacks_mu;
     int want_form = B2_FORM_AUTO, want_split = 0;  // the 2D launch that the caller asked for
     // F16 form: the filter's FP32 rows before they become FP16 quads, and the device words
     // (max |y| as bits, inverse scale) of the quads' power-of-two scale
@@ -111,6 +113,7 @@ struct sgb_plan {
     ~sgb_plan() {
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
+        if (stacks) cudaMemPoolDestroy(stacks);
     }
     void mark(int i, cudaStream_t st) {
         if (timing) cudaEventRecord(ev[i], st);
@@ -721,18 +724,37 @@ int sgb_fdk(sgb_plan *P, const float *proj, float *image, int flags, void *strea
     return plan_done(P, flags, st);
 }
 
-// Room for n bytes in a workspace that the call can do without: not grown while the stream is being
-// captured, nor past the device's memory.
-static bool grow_between_captures(DevBuf &b, size_t n, cudaStream_t st) {
-    if (b.p && n <= b.bytes) return true;
+// n bytes for one call's interleaved slices, in the order of its stream (to be freed with cudaFreeAsync),
+// or null: a call can do without.  A plan's back-projection may run on several streams and threads at a
+// time, so a call has a block of its own, from a pool that keeps its memory until the plan is destroyed.
+// A captured call has none: its graph may be replayed beside any other call.
+static float *stack_buffer(sgb_plan *P, size_t n, cudaStream_t st) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
-        return false;
+        return nullptr;
     }
-    if (b.reserve(n) == SGB_OK) return true;
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(P->stacks_mu);
+        if (!P->stacks) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            uint64_t keep = UINT64_MAX;
+            if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            P->stacks = pool;
+        }
+        pool = P->stacks;
+    }
+    void *p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, n, pool, st) == cudaSuccess) return static_cast<float *>(p);
     cudaGetLastError();
-    return false;
+    return nullptr;
 }
 
 // A 2D plan's back-projection of nslices, but for the launch's choice and the buffers.
@@ -769,17 +791,19 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
     Back2Args A = back2_args(P, nslices);
     A.sino = sino;
     A.image = image;
-    const Back2Args all = A;
+    Back2Args one = A;
     back2_choose(A, true);
     if (A.sl == 4) {
         const long long n = (long long)g.nb * g.na;
-        if (grow_between_captures(P->inter, sizeof(float) * 4 * n * floor_div_up(nslices, 4), st)) {
-            SGB_TRY(launch_interleave4(sino, P->inter.as<float>(), n, nslices, st));
-            A.sino4 = P->inter.as<float>();
-        } else {  // slice by slice
-            A = all;
-            back2_choose(A, false);
+        if (float *four = stack_buffer(P, sizeof(float) * 4 * n * floor_div_up(nslices, 4), st)) {
+            int s = launch_interleave4(sino, four, n, nslices, st);
+            A.sino4 = four;
+            if (s == SGB_OK) s = launch_back2(A, st);
+            SGB_CUDA(cudaFreeAsync(four, st));
+            return s;
         }
+        back2_choose(one, false);
+        return launch_back2(one, st);
     }
     return launch_back2(A, st);
 }
