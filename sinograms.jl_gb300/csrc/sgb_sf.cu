@@ -22,9 +22,10 @@
 //     coordinates across and along the central ray from the source), so the trapezoid keeps FP32
 //     relative accuracy where uc is ~1e3 bins;
 //   * both kernels evaluate footprints and elements with the same explicitly rounded FP32 operations
-//     (__fmaf_rn and friends cannot be contracted differently in the two kernels), so each element
-//     has the same bits in both and the back-projector is the transpose of the forward projector up
-//     to summation order;
+//     (__fmaf_rn and friends cannot be contracted differently in the two kernels), and an element that
+//     serves several views and pixels at the same one of them (SfItem), so each element has the same
+//     bits in both and the back-projector is the transpose of the forward projector up to summation
+//     order;
 //   * forward: one thread per detector bin and one CTA per (view, chunk of bins).  The CTA sweeps the
 //     image lines (rows, or columns when the view's rays cross columns more steeply or the source
 //     lies within the rows' range); per line it computes into shared memory the footprints of the
@@ -36,7 +37,8 @@
 //     have the same elements in the views that see them alike, at the same bins or at those mirrored about
 //     the detector's centre.  So the forward kernel sums a view's bins over the image together with the
 //     bins of the views that are its images, over the image's images, and the back-projector takes a pixel
-//     with its images: each element is evaluated once for two or four.
+//     with its images: each element is evaluated once for two or four.  Mirrored elements agree to rounding
+//     only (wb + K a and wb - K a round differently): both evaluate them at the forward sweep's view.
 // Both directions are bound by issue, most of it the elements.  888 x 90 arc, 512^2: forward 437 -> 136 us,
 // back 242 -> 115 us with four slots against one element at a time; a pair of calls 683 -> 264 us.
 // Plans compute the per-view constants and the boundary-ray table once, in FP64 on the device.
@@ -79,7 +81,8 @@ struct SfView {
     float p3, ph, phr01, phr23;  // ... its amplitude and trapezoid constants
     float pc3;
     int rows;                    // forward sweep: 1 = rows (lines of constant y), 0 = columns
-    int pad0, pad1;
+    int map;                     // back: the item's pixel
+    int pad;
 };
 static_assert(sizeof(SfView) == 80, "SfView layout");
 
@@ -87,17 +90,30 @@ static_assert(sizeof(SfView) == 80, "SfView layout");
 struct SfArgs {
     int nb, na, nx, ny;
     int splits;  // forward: the image lines are split over this many CTAs per (view, chunk of bins)
-    int gsplit;  // back: CTAs of a cluster that share a tile's views
+    int gsplit;  // back: CTAs of a cluster that share a tile's items
+    int nitem;   // back: items
     int nrep;    // forward: views that are not images of others
     ScanSlots sym;
     float wb, ax, ay, axy, hx, hy;
 };
 
 // A view and its images in the slots: entry j is slot j's view, kSfRev if its bins run the other way,
-// kSfDup if an earlier slot has the same view.
+// kSfDup if an earlier slot has the same view.  The forward projector evaluates a view's elements at the
+// first view of its images (its representative), in the slot that the view has there.
 constexpr int kSfRev = 1 << 30, kSfDup = 1 << 29, kSfView = kSfDup - 1;
 
-// One pixel's footprint in one view, relative to uc.
+// What the back-projector takes at a time: for the view w that slot j gives a view v, and slot j's image of
+// its pixel, the element that the forward projector evaluates: w's representative `rep` sees it at the pixel
+// that `map` (as ScanSlots::Slot::map) gives for the thread's.  `rows`: w per slot, kSfRev if the element's
+// bins run the other way there; kSfDup where the slot's element lies at another pixel, in another item (an
+// item per view but for views that are their own images: two).
+struct SfItem {
+    int4 rows;
+    int rep, map;
+};
+
+// One pixel's footprint in one view, relative to uc: the bin coordinate of the centre (parallel beams: less
+// wb, so that a half turn of the pixel negates it exactly).
 struct SfRec {
     float uc, d0, d1, d2, d3, hr01, hr23, c3, h;
 };
@@ -132,11 +148,28 @@ __host__ __device__ __forceinline__ void sf_finish(SfRec &r, float o0, float o1,
 #endif
 }
 
+// The trapezoid's running integral from its centre or its start.  Parallel beams: symmetric (d0 = -d3,
+// d1 = -d2), and evaluated as the odd function that it is, so that a pixel and its half turn have the same
+// elements at mirrored bins, in every bit.
+template <int GEO>
 __device__ __forceinline__ float sf_cdf(float b, const SfRec &r) {
+    if (GEO == 0) {
+        const float a = __fsub_rn(fminf(fmaxf(b, r.d0), r.d1), r.d0);
+        const float z = __fsub_rn(r.d3, fminf(fmaxf(b, r.d2), r.d3));
+        const float p = __fmul_rn(__fmul_rn(r.hr01, a), a), q = __fmul_rn(__fmul_rn(r.hr23, z), z);
+        return __fadd_rn(fminf(fmaxf(b, r.d1), r.d2), __fsub_rn(p, q));
+    }
     const float a = __fsub_rn(fminf(fmaxf(b, r.d0), r.d1), r.d0);
     const float m = __fsub_rn(fminf(fmaxf(b, r.d1), r.d2), r.d1);
     const float z = __fsub_rn(r.d3, fminf(fmaxf(b, r.d2), r.d3));
     return __fadd_rn(__fmaf_rn(__fmul_rn(r.hr01, a), a, m), __fmaf_rn(-__fmul_rn(r.hr23, z), z, r.c3));
+}
+
+// The lower boundary of bin k, from where uc counts (exact where wb is a multiple of 1/4).
+template <int GEO>
+__device__ __forceinline__ float sf_bound(int k, const SfArgs &A) {
+    const float b = (float)k - 0.5f;
+    return GEO == 0 ? __fsub_rn(b, A.wb) : b;
 }
 
 // Footprint of the pixel centred at (xc, yc).  GEO: 0 parallel, 1 arc, 2 flat.
@@ -144,7 +177,7 @@ template <int GEO>
 __device__ __forceinline__ SfRec sf_pixel(const SfView &V, const SfArgs &A, float xc, float yc) {
     SfRec r;
     if (GEO == 0) {
-        r.uc = __fmaf_rn(__fmaf_rn(xc, V.cb, __fmul_rn(yc, V.sb)), V.K, A.wb);
+        r.uc = __fmul_rn(__fmaf_rn(xc, V.cb, __fmul_rn(yc, V.sb)), V.K);
         r.d0 = V.p0;
         r.d1 = V.p1;
         r.d2 = V.p2;
@@ -332,8 +365,8 @@ __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const
     const float2 cl = R[k0], ch = R[kend];
     const bool active = ka < A.nb;
     const float2 bl = R[min(ka, A.nb)], bh = R[max(kb, 0)];
-    // boundaries of bins ka and ka + 1 (exact in FP32, as the back-projector forms them)
-    const float e0 = (float)ka - 0.5f, e1 = (float)ka + 0.5f, e2 = (float)(ka + 1) + 0.5f;
+    // boundaries of bins ka and ka + 1 (as the back-projector forms them)
+    const float e0 = sf_bound<GEO>(ka, A), e1 = sf_bound<GEO>(ka + 1, A), e2 = sf_bound<GEO>(ka + 2, A);
     const int per = (nln + A.splits - 1) / A.splits, jb = blockIdx.z * per, je = min(nln, jb + per);
     float acc0[NS] = {}, acc1[NS] = {};
     // A pass is at most CAP pixels of a line: [p0, p1] of line j, whose wedge ends at ib.  The next
@@ -435,8 +468,8 @@ __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const
                 r.hr23 = a1.z;
                 r.c3 = a1.w;
             }
-            const float g0 = sf_cdf(__fsub_rn(e0, r.uc), r), g1 = sf_cdf(__fsub_rn(e1, r.uc), r);
-            const float g2 = sf_cdf(__fsub_rn(e2, r.uc), r);
+            const float g0 = sf_cdf<GEO>(__fsub_rn(e0, r.uc), r), g1 = sf_cdf<GEO>(__fsub_rn(e1, r.uc), r);
+            const float g2 = sf_cdf<GEO>(__fsub_rn(e2, r.uc), r);
             const float w0 = __fmul_rn(h, __fsub_rn(g1, g0)), w1 = __fmul_rn(h, __fsub_rn(g2, g1));
 #pragma unroll
             for (int s = 0; s < NS; s++) {
@@ -469,16 +502,27 @@ __global__ void sf_sum_splits(const float *__restrict__ part, int splits, long l
 }
 
 // ------------------------------------------------------------------- back
+// The items' view constants, in order.
+__global__ void sf_item_views(const SfItem *items, int n, const SfView *views, SfView *out, int4 *rows) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    out[i] = views[items[i].rep];
+    out[i].map = items[i].map;
+    rows[i] = items[i].rows;
+}
+
 template <int GEO, int NS>
 __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, const SfView *__restrict__ views,
                                                                    const float *__restrict__ xcs,
                                                                    const float *__restrict__ ycs,
                                                                    const float *__restrict__ sino,
                                                                    const uint8_t *__restrict__ mask,
-                                                                   const int4 *__restrict__ images,
+                                                                   const int4 *__restrict__ rows,
+                                                                   const float *__restrict__ zeros,
                                                                    float *__restrict__ image) {
     __shared__ SfView sv[kViewChunk];
-    __shared__ int4 si[kViewChunk];
+    __shared__ __align__(16) const float *sp[kViewChunk][NS];  // bin 0 of the slots' rows, and the way their bins run
+    __shared__ __align__(16) int ss[kViewChunk][NS];
     __shared__ float part[NS][kBackTx * kBackTy];
     const int tid = threadIdx.x + kBackTx * threadIdx.y, rank = blockIdx.z;
     const int px = blockIdx.x * kBackTx + threadIdx.x, py = blockIdx.y * kBackTy + threadIdx.y;
@@ -489,8 +533,10 @@ __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, con
         own[s] = slot_pixel(A.sym, A.nx, A.ny, s, px, py, &n[s]);
         on |= own[s] && (!mask || mask[n[s]]);
     }
-    const float xc = px < A.nx ? xcs[px] : 0.f, yc = py < A.ny ? ycs[py] : 0.f;
-    const int va = (int)((long long)A.na * rank / A.gsplit), vb = (int)((long long)A.na * (rank + 1) / A.gsplit);
+    const int cx = min(px, A.nx - 1), cy = min(py, A.ny - 1);
+    float xc = xcs[cx], yc = ycs[cy];
+    int map = 0;  // of (xc, yc)
+    const int va = (int)((long long)A.nitem * rank / A.gsplit), vb = (int)((long long)A.nitem * (rank + 1) / A.gsplit);
     float acc[NS] = {};
     for (int v0 = va; v0 < vb; v0 += kViewChunk) {
         const int nv = min(kViewChunk, vb - v0);
@@ -498,27 +544,39 @@ __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, con
         const int *src = reinterpret_cast<const int *>(views + v0);
         int *dst = reinterpret_cast<int *>(sv);
         for (int t = tid; t < nv * (int)(sizeof(SfView) / 4); t += kBackTx * kBackTy) dst[t] = __ldg(src + t);
-        if (tid < nv) si[tid] = images[v0 + tid];
+        static_assert(kViewChunk * NS <= kBackTx * kBackTy, "a thread stages one slot of one item");
+        if (tid < nv * NS) {
+            const int e = __ldg(reinterpret_cast<const int *>(rows + v0 + tid / NS) + tid % NS);
+            sp[tid / NS][tid % NS] = e & kSfDup ? zeros : sino + (size_t)A.nb * (e & kSfView) + (e & kSfRev ? A.nb - 1 : 0);
+            ss[tid / NS][tid % NS] = e & kSfRev ? -1 : 1;
+        }
         __syncthreads();
         if (!on) continue;
         for (int vv = 0; vv < nv; vv++) {
+            if (NS > 1 && sv[vv].map != map) {  // a few times per call: the items' maps come in runs
+                map = sv[vv].map;
+                int qx = map & 4 ? cy : cx, qy = map & 4 ? cx : cy;
+                if (map & 1) qx = A.nx - 1 - qx;
+                if (map & 2) qy = A.ny - 1 - qy;
+                xc = __ldg(xcs + qx);
+                yc = __ldg(ycs + qy);
+            }
             const SfRec r = sf_pixel<GEO>(sv[vv], A, xc, yc);
-            const float lo = __fadd_rn(r.uc, r.d0) - 0.5f, hi = __fadd_rn(r.uc, r.d3) + 0.5f;
+            const float uc = GEO == 0 ? __fadd_rn(r.uc, A.wb) : r.uc;
+            const float lo = __fadd_rn(uc, r.d0) - 0.5f, hi = __fadd_rn(uc, r.d3) + 0.5f;
             const int kf = max(0, (int)ceilf(fminf(fmaxf(lo, -1.f), (float)A.nb)));
             const int kl = min(A.nb - 1, (int)floorf(fminf(fmaxf(hi, -1.f), (float)A.nb)));
             if (kf > kl) continue;
-            const int4 im = si[vv];
-            const int iv[4] = {im.x, im.y, im.z, im.w};
             const float *row[NS];
             int step[NS];
 #pragma unroll
             for (int s = 0; s < NS; s++) {
-                step[s] = iv[s] & kSfRev ? -1 : 1;
-                row[s] = sino + (size_t)A.nb * (iv[s] & kSfView) + (iv[s] & kSfRev ? A.nb - 1 - kf : kf);
+                step[s] = NS == 1 ? 1 : ss[vv][s];
+                row[s] = sp[vv][s] + step[s] * kf;
             }
-            float gprev = sf_cdf(__fsub_rn((float)kf - 0.5f, r.uc), r);
+            float gprev = sf_cdf<GEO>(__fsub_rn(sf_bound<GEO>(kf, A), r.uc), r);
             for (int k = kf; k <= kl; k++) {
-                const float g = sf_cdf(__fsub_rn((float)k + 0.5f, r.uc), r);
+                const float g = sf_cdf<GEO>(__fsub_rn(sf_bound<GEO>(k + 1, A), r.uc), r);
                 const float w = __fmul_rn(r.h, __fsub_rn(g, gprev));
 #pragma unroll
                 for (int s = 0; s < NS; s++) {
@@ -553,7 +611,7 @@ __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, con
 
 template <int GEO, int NS>
 int sf_launch_back(const SfArgs &A, const SfView *views, const float *xcs, const float *ycs, const float *sino,
-                   const uint8_t *mask, const int4 *images, float *image, cudaStream_t st) {
+                   const uint8_t *mask, const int4 *rows, const float *zeros, float *image, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((A.sym.hx + kBackTx - 1) / kBackTx, (A.sym.hy + kBackTy - 1) / kBackTy, A.gsplit);
     cfg.blockDim = dim3(kBackTx, kBackTy);
@@ -565,7 +623,7 @@ int sf_launch_back(const SfArgs &A, const SfView *views, const float *xcs, const
     attr[0].val.clusterDim.z = A.gsplit;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, sf_back_kernel<GEO, NS>, A, views, xcs, ycs, sino, mask, images, image);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, sf_back_kernel<GEO, NS>, A, views, xcs, ycs, sino, mask, rows, zeros, image);
     if (e != cudaSuccess) {
         set_error("sf_back_kernel: launch failed: %s", cudaGetErrorString(e));
         return SGB_ERR_CUDA;
@@ -575,14 +633,18 @@ int sf_launch_back(const SfArgs &A, const SfView *views, const float *xcs, const
 
 // One slot count of a direction, for the plan's geometry kind.
 template <int NS>
-int sf_launch(int kind, bool forward, const SfArgs &A, const SfView *views, const float2 *rays, const float *xcs,
-              const float *ycs, const float *src, const float *srct, const uint8_t *mask, const int4 *reps, const int4 *images, float *dst,
-              cudaStream_t st) {
-    if (!forward) {
-        if (kind == SGB_PAR) return sf_launch_back<0, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
-        if (kind == SGB_ARC) return sf_launch_back<1, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
-        return sf_launch_back<2, NS>(A, views, xcs, ycs, src, mask, images, dst, st);
-    }
+int sf_launch_back_kind(int kind, const SfArgs &A, const SfView *views, const float *xcs, const float *ycs,
+                        const float *sino, const uint8_t *mask, const int4 *rows, const float *zeros, float *image,
+                        cudaStream_t st) {
+    if (kind == SGB_PAR) return sf_launch_back<0, NS>(A, views, xcs, ycs, sino, mask, rows, zeros, image, st);
+    if (kind == SGB_ARC) return sf_launch_back<1, NS>(A, views, xcs, ycs, sino, mask, rows, zeros, image, st);
+    return sf_launch_back<2, NS>(A, views, xcs, ycs, sino, mask, rows, zeros, image, st);
+}
+
+template <int NS>
+int sf_launch_forward(int kind, const SfArgs &A, const SfView *views, const float2 *rays, const float *xcs,
+                      const float *ycs, const float *src, const float *srct, const int4 *reps, float *dst,
+                      cudaStream_t st) {
     const dim3 grid((A.nb + kFwdBins - 1) / kFwdBins, A.nrep, A.splits);
     if (kind == SGB_PAR)
         sf_project_kernel<0, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
@@ -605,7 +667,8 @@ struct sgb_sf_plan {
     SfGeo G{};
     SfArgs A{};
     DevBuf betas, views, rays, axes, mask, din, dout, part, img;
-    DevBuf images;  // every view's images (na), then the representative views' (nrep)
+    DevBuf reps;  // forward: the representative views' images
+    DevBuf item_views, item_rows, zeros;  // back: the items' constants and rows; a row of zeros
     const uint8_t *mask_dev = nullptr;
 };
 
@@ -660,6 +723,72 @@ int sf_geometry(const sgb_sino_geom *rg, const sgb_image_geom *ig, SfGeo *G) {
     return SGB_OK;
 }
 
+// The pixel whose image in slot b is the thread's pixel's image in slot a, as a map (Slot::map) of the
+// thread's: slot a's map, then the inverse of slot b's.
+int sf_map_between(int a, int b) {
+    auto apply = [](int f, int x, int y, int *u, int *v) {
+        *u = f & 4 ? y : x;
+        *v = f & 4 ? x : y;
+        if (f & 1) *u = -*u;
+        if (f & 2) *v = -*v;
+    };
+    for (int f = 0; f < 8; f++) {  // b after f is a, on a point without symmetry
+        int x, y, u, v, p, q;
+        apply(f, 1, 2, &x, &y);
+        apply(b, x, y, &u, &v);
+        apply(a, 1, 2, &p, &q);
+        if (u == p && v == q) return f;
+    }
+    return 0;
+}
+
+// The representative views' images, and the back-projector's items.  `half`: a half turn of the pixel gives the
+// same elements at mirrored bins (parallel beams, centred detector and image), so that it needs no item.
+void sf_items(const ScanSlots &S, int na, bool half, std::vector<int4> &reps, std::vector<SfItem> &items) {
+    struct Own {
+        int rep, slot;
+        bool rev;
+    };
+    std::vector<Own> own(na, Own{-1, 0, false});
+    for (int v = 0; v < na; v++) {
+        if (own[v].rep >= 0) continue;
+        int e[4] = {v, 0, 0, 0};
+        own[v] = {v, 0, false};
+        for (int j = 1; j < S.ns; j++) {
+            bool rev;
+            const int u = slot_view(S, na, j, v, &rev);
+            e[j] = u | (rev ? kSfRev : 0);
+            if (own[u].rep >= 0) e[j] |= kSfDup;
+            else own[u] = {v, j, rev};
+        }
+        reps.push_back(make_int4(e[0], e[1], e[2], e[3]));
+    }
+    for (int v = 0; v < na; v++) {
+        int row[4], map[4], rep[4];
+        for (int j = 0; j < S.ns; j++) {
+            bool rev;
+            const int w = slot_view(S, na, j, v, &rev);
+            row[j] = w | (own[w].rev ? kSfRev : 0);
+            rep[j] = own[w].rep;
+            // the representative sees slot j's image of the pixel where w's slot takes it from
+            map[j] = sf_map_between(S.slot[j].map, S.slot[own[w].slot].map);
+            if (half && map[j] & 2) {
+                map[j] ^= 3;
+                row[j] ^= kSfRev;
+            }
+        }
+        for (int j = 0; j < S.ns; j++) {
+            bool first = true;
+            for (int i = 0; i < j; i++) first &= rep[i] != rep[j] || map[i] != map[j];
+            if (!first) continue;
+            int e[4] = {kSfDup, kSfDup, kSfDup, kSfDup};
+            for (int i = j; i < S.ns; i++)
+                if (rep[i] == rep[j] && map[i] == map[j]) e[i] = row[i];
+            items.push_back(SfItem{make_int4(e[0], e[1], e[2], e[3]), rep[j], map[j]});
+        }
+    }
+}
+
 // Line splits of the forward projector: enough CTAs for about two resident waves of four-warp
 // CTAs (16 per SM), at most 32 and at least 8 image lines per CTA.
 int sf_default_splits(const SfGeo &G, int nrep) {
@@ -688,13 +817,6 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
     const float *xcs = P->axes.as<float>(), *ycs = xcs + G.nx;
     const SfView *views = P->views.as<SfView>();
     const float *src = static_cast<const float *>(in_dev);
-    const int4 *images = P->images.as<int4>();
-    auto run = [&](bool fwd, float *dst) {
-        const float2 *rays = P->rays.as<float2>();
-        auto go = P->A.sym.ns == 4 ? sf_launch<4> : (P->A.sym.ns == 2 ? sf_launch<2> : sf_launch<1>);
-        return go(G.kind, fwd, P->A, views, rays, xcs, ycs, fwd ? P->img.as<float>() : src, P->img.as<float>() + nimg, P->mask_dev,
-                  images + G.na, images, dst, st);
-    };
     if (forward) {
         const int splits = P->A.splits;
         static_assert(kFwdBpt == 2, "sf_project_kernel accumulates two bins per thread");
@@ -706,13 +828,19 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
         sf_image_kernel<<<dim3((G.nx + 31) / 32, (G.ny + 31) / 32), dim3(32, 8), 0, st>>>(
             src, P->mask_dev, G.nx, G.ny, P->img.as<float>(), P->img.as<float>() + nimg);
         SGB_TRY(after_launch("sf_image_kernel"));
-        SGB_TRY(run(true, dst));
+        auto go = P->A.sym.ns == 4 ? sf_launch_forward<4>
+                                   : (P->A.sym.ns == 2 ? sf_launch_forward<2> : sf_launch_forward<1>);
+        SGB_TRY(go(G.kind, P->A, views, P->rays.as<float2>(), xcs, ycs, P->img.as<float>(), P->img.as<float>() + nimg,
+                   P->reps.as<int4>(), dst, st));
         if (splits > 1) {
             sf_sum_splits<<<(unsigned)((nsino + 255) / 256), 256, 0, st>>>(dst, splits, (long long)nsino, out_dev);
             SGB_TRY(after_launch("sf_sum_splits"));
         }
     } else {
-        SGB_TRY(run(false, out_dev));
+        auto go = P->A.sym.ns == 4 ? sf_launch_back_kind<4>
+                                   : (P->A.sym.ns == 2 ? sf_launch_back_kind<2> : sf_launch_back_kind<1>);
+        SGB_TRY(go(G.kind, P->A, P->item_views.as<SfView>(), xcs, ycs, src, P->mask_dev, P->item_rows.as<int4>(),
+                   P->zeros.as<float>(), out_dev, st));
     }
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(out, out_dev, nout * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -764,26 +892,21 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
     A.hy = (float)(0.5 * std::fabs(G.dy));
     A.sym = scan_slots(rg->kind, G.na, G.nx, G.ny, 2 * G.wb == G.nb - 1.0, G.so == 0, rg->orbit, rg->orbit_start, ig->deltas,
                        ig->offsets, false);
-    // every view's images, and those of the views that no earlier one's images include
-    std::vector<int4> images(G.na), reps;
-    std::vector<char> seen(G.na, 0);
-    for (int v = 0; v < G.na; v++) {
-        int e[4] = {v, 0, 0, 0};
-        for (int j = 1; j < A.sym.ns; j++) {
-            bool rev;
-            const int u = slot_view(A.sym, G.na, j, v, &rev);
-            e[j] = u | (rev ? kSfRev : 0);
-            for (int i = 0; i < j; i++)
-                if ((e[i] & kSfView) == u) e[j] |= kSfDup;
-        }
-        images[v] = make_int4(e[0], e[1], e[2], e[3]);
-        if (!seen[v]) reps.push_back(images[v]);
-        for (int j = 0; j < A.sym.ns; j++) seen[e[j] & kSfView] = 1;
-    }
+    std::vector<int4> reps;
+    std::vector<SfItem> items;
+    const bool centred = 2 * G.wb == G.nb - 1.0;
+    sf_items(A.sym, G.na, G.kind == SGB_PAR && centred && G.ox == 0 && G.oy == 0, reps, items);
     A.nrep = (int)reps.size();
-    images.insert(images.end(), reps.begin(), reps.end());
-    SGB_TRY(P->images.reserve(sizeof(int4) * images.size()));
-    SGB_CUDA(cudaMemcpyAsync(P->images.p, images.data(), sizeof(int4) * images.size(), cudaMemcpyHostToDevice, st));
+    A.nitem = (int)items.size();
+    DevBuf items_dev;
+    SGB_TRY(P->reps.reserve(sizeof(int4) * reps.size()));
+    SGB_CUDA(cudaMemcpyAsync(P->reps.p, reps.data(), sizeof(int4) * reps.size(), cudaMemcpyHostToDevice, st));
+    SGB_TRY(items_dev.reserve(sizeof(SfItem) * items.size()));
+    SGB_CUDA(cudaMemcpyAsync(items_dev.p, items.data(), sizeof(SfItem) * items.size(), cudaMemcpyHostToDevice, st));
+    SGB_TRY(P->item_views.reserve(sizeof(SfView) * items.size()));
+    SGB_TRY(P->item_rows.reserve(sizeof(int4) * items.size()));
+    SGB_TRY(P->zeros.reserve(sizeof(float) * G.nb));
+    SGB_CUDA(cudaMemsetAsync(P->zeros.p, 0, sizeof(float) * G.nb, st));
     A.splits = sf_default_splits(G, A.nrep);
     // back: about four CTAs of 256 pixels per SM, at least 8 views each
     const long long tiles = (long long)((A.sym.hx + kBackTx - 1) / kBackTx) * ((A.sym.hy + kBackTy - 1) / kBackTy);
@@ -792,6 +915,9 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
     SGB_TRY(P->rays.reserve(sizeof(float2) * (size_t)G.na * (G.nb + 1)));
     sf_setup_views<<<(G.na + 127) / 128, 128, 0, st>>>(G, P->betas.as<double>(), P->views.as<SfView>());
     SGB_TRY(after_launch("sf_setup_views"));
+    sf_item_views<<<(A.nitem + 127) / 128, 128, 0, st>>>(items_dev.as<SfItem>(), A.nitem, P->views.as<SfView>(),
+                                                        P->item_views.as<SfView>(), P->item_rows.as<int4>());
+    SGB_TRY(after_launch("sf_item_views"));
     const long long nr = (long long)G.na * (G.nb + 1);
     sf_setup_rays<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(G, P->betas.as<double>(), P->views.as<SfView>(),
                                                                    P->rays.as<float2>());
