@@ -94,7 +94,16 @@ struct sgb_plan {
     DevBuf in_buf, filt_buf, img_buf;
     // 2D stacks: where a call's interleaved slices come from (stack_buffer)
     cudaMemPool_t stacks = nullptr;
-    std::mutex stacks_mu;
+    // 2D launches chosen so far (back2_launch)
+    struct {
+        int nslices;
+        bool fours;
+        Back2Args A;
+    } launches[8];
+    int nlaunches = 0;
+    std::mutex back2_mu;  // stacks and launches
+    float wanted = 1.f;  // share of a 2D image's tiles that have a pixel inside the mask
+    double reach = 1e30;  // and how far from the centre such pixels lie, in bins
     int want_form = B2_FORM_AUTO, want_split = 0;  // the 2D launch that the caller asked for
     // F16 form: the filter's FP32 rows before they become FP16 quads, and the device words
     // (max |y| as bits, inverse scale) of the quads' power-of-two scale
@@ -192,6 +201,9 @@ int plan_image(sgb_plan *P, const sgb_image_geom *ig, double ds, int ndim, cudaS
         std::vector<double> z = image_axis(P->nz, ig->deltas[2], ig->offsets[2], ds);
         SGB_TRY(upload_f32(z.data(), z.size(), 1.0, P->zds, st));
     }
+    if (ndim == 2 && ig->mask) 
+        P->wanted = back2_wanted(ig->mask, P->nx, P->ny, ig->deltas[0] / ds, ig->deltas[1] / ds, ig->offsets[0], ig->offsets[1],
+                                 &P->reach);
     return upload_mask(ig->mask, (size_t)P->nx * P->ny * P->nz, P->mask, &P->mask_dev, st);
 }
 
@@ -736,7 +748,7 @@ static float *stack_buffer(sgb_plan *P, size_t n, cudaStream_t st) {
     }
     cudaMemPool_t pool;
     {
-        std::lock_guard<std::mutex> lock(P->stacks_mu);
+        std::lock_guard<std::mutex> lock(P->back2_mu);
         if (!P->stacks) {
             cudaMemPoolProps props = {};
             props.allocType = cudaMemAllocationTypePinned;
@@ -776,23 +788,34 @@ static Back2Args back2_args(const sgb_plan *P, int nslices) {
     A.dsd_ds = (float)(g.dsd / g.d);
     A.dso_ds = (float)((g.dsd - g.dod) / g.d);
     A.so_ds = (float)(g.source_offset / g.d);
-    back2_window(A, P->deltas[0] / g.d, P->deltas[1] / g.d);
+    back2_window(A, P->deltas[0] / g.d, P->deltas[1] / g.d, P->reach);
     A.sym = scan_slots(g.kind, g.na, P->nx, P->ny, 2.0 * A.wb == g.nb + 1.0, g.source_offset == 0, g.orbit, g.orbit_start,
                        P->deltas, P->offsets, true);
     A.nslices = nslices;
+    A.wanted = P->wanted;
     A.want_form = P->want_form;
     A.want_split = P->want_split;
+    return A;
+}
+
+// The launch for nslices; `fours`: the caller has room for interleaved slices.  The geometry decides it, so a
+// plan keeps the first few (choosing takes 3 us on the host, as long as a launch).
+static Back2Args back2_launch(sgb_plan *P, int nslices, bool fours) {
+    std::lock_guard<std::mutex> lock(P->back2_mu);
+    for (int i = 0; i < P->nlaunches; i++)
+        if (P->launches[i].nslices == nslices && P->launches[i].fours == fours) return P->launches[i].A;
+    Back2Args A = back2_args(P, nslices);
+    back2_choose(A, fours);
+    if (P->nlaunches < (int)std::size(P->launches)) P->launches[P->nlaunches++] = {nslices, fours, A};
     return A;
 }
 
 // Back-projection of a 2D plan's filtered slices.
 static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices, cudaStream_t st) {
     const sgb_sino_geom &g = P->sg;
-    Back2Args A = back2_args(P, nslices);
+    Back2Args A = back2_launch(P, nslices, true);
     A.sino = sino;
     A.image = image;
-    Back2Args one = A;
-    back2_choose(A, true);
     if (A.sl == 4) {
         const long long n = (long long)g.nb * g.na;
         if (float *four = stack_buffer(P, sizeof(float) * 4 * n * floor_div_up(nslices, 4), st)) {
@@ -802,8 +825,9 @@ static int plan_back2(sgb_plan *P, const float *sino, float *image, int nslices,
             SGB_CUDA(cudaFreeAsync(four, st));
             return s;
         }
-        back2_choose(one, false);
-        return launch_back2(one, st);
+        A = back2_launch(P, nslices, false);
+        A.sino = sino;
+        A.image = image;
     }
     return launch_back2(A, st);
 }
@@ -812,8 +836,10 @@ int sgb_plan_set_back_form(sgb_plan *P, int form, int split) {
     SGB_REQUIRE(P && !P->ct, "plan_set_back_form: needs a 2D plan");
     SGB_REQUIRE(form >= B2_FORM_AUTO && form <= B2_FORM_FOURS, "plan_set_back_form: unknown form %d", form);
     SGB_REQUIRE(split >= 0 && split <= 8, "plan_set_back_form: split must be in [0, 8], got %d", split);
+    std::lock_guard<std::mutex> lock(P->back2_mu);
     P->want_form = form;
     P->want_split = split;
+    P->nlaunches = 0;
     return SGB_OK;
 }
 
@@ -1035,9 +1061,10 @@ static int back2_seam(float *image, const float *sino, int nb, int na, const dou
     A.dso_ds = (float)(dso / ds);
     A.so_ds = (float)(source_offset / ds);
     A.sym = ScanSlots{1, nx, ny, 0, 0, {{0, 1, 0, 0}}};
+    A.wanted = 1.f;
     A.want_form = B2_FORM_AUTO;
     // the axes are the caller's, spaced as they like: their mean spacing
-    back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0);
+    back2_window(A, nx > 1 ? (xc[nx - 1] - xc[0]) / ds / (nx - 1) : 0, ny > 1 ? (yc[ny - 1] - yc[0]) / ds / (ny - 1) : 0, 1e30);
     back2_choose(A, false);
     SGB_TRY(launch_back2(A, st));
     if (!(flags & SGB_DEVICE_PTRS))

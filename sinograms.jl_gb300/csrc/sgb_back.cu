@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 namespace sgb {
 
@@ -163,13 +164,38 @@ int launch_fdk_back(const FdkArgs &A, cudaStream_t st) {
                     : (geo == 1 ? launch_fdk_z<float, 1>(A, st) : launch_fdk_z<float, 0>(A, st));
 }
 
-// Staged bins per segment: what a 32 x 32 tile of dx x dy pixels (in bins) spans at most, with the kernel's
-// margins; a tile nearer the source than the image's edge midpoints may span more and reads global memory.
-void back2_window(Back2Args &A, double dx, double dy) {
-    const double r = std::max(std::fabs(dx) * A.nx, std::fabs(dy) * A.ny) / 2;
+// Staged bins per segment: what a 32 x 32 tile of dx x dy pixels (in bins) with pixels within `reach` (in bins)
+// of the centre spans at most, with the kernel's margins; tiles that span more read global memory.
+void back2_window(Back2Args &A, double dx, double dy, double reach) {
+    const double corner = std::hypot(dx * A.nx, dy * A.ny) / 2, r = std::min(corner, reach + 32 * std::hypot(dx, dy));
     const double mag = A.mode == SGB_PAR ? 1.0 : A.dsd_ds / std::max(1e-3, A.dso_ds - r);
     const double span = 1.05 * mag * 31 * std::hypot(dx, dy) + 10;
     A.w = span < 256 ? ((int)span + 7) / 8 * 8 : 256;
+}
+
+float back2_wanted(const uint8_t *mask, int nx, int ny, double dx, double dy, double ox, double oy, double *reach) {
+    const int tx = floor_div_up(nx, kB2X), ty = floor_div_up(ny, kB2Y * kB2P);
+    std::vector<char> in((size_t)tx * ty, 0);
+    double far = 0;
+    for (int y = 0; y < ny; y++) {
+        const uint8_t *row = mask + (size_t)nx * y;
+        int first = 0, last = nx - 1;  // the row's ends, the farthest of its pixels
+        while (first < nx && !row[first]) first++;
+        if (first == nx) continue;
+        while (!row[last]) last--;
+        const double v = dy * (y - ((ny - 1) / 2.0 + oy));
+        for (int x : {first, last}) {
+            const double u = dx * (x - ((nx - 1) / 2.0 + ox));
+            far = std::max(far, u * u + v * v);
+        }
+        char *tiles = in.data() + (size_t)tx * (y / (kB2Y * kB2P));
+        for (int t = first / kB2X; t <= last / kB2X; t++)
+            for (int x = std::max(first, t * kB2X); !tiles[t] && x <= last && x < (t + 1) * kB2X; x++) tiles[t] = row[x] != 0;
+    }
+    *reach = std::sqrt(far);
+    size_t n = 0;
+    for (char c : in) n += c;
+    return (float)n / (float)in.size();
 }
 
 // Which pixels and views share geometry: needs the grid centred (offsets 0) on the axes that a slot
@@ -231,38 +257,55 @@ ScanSlots scan_slots(int kind, int na, int nx, int ny, bool centred, bool source
 }
 
 void back2_choose(Back2Args &A, bool fours) {
-    // Predicted time in us.  A view of a tile takes a thread its pixels' geometry and taps (instructions)
-    // and the staging; a CTA's 8 warps issue 2.8 per clock between them when the SM has enough CTAs, and
-    // a CTA alone takes 2.4 times its share.  Starting, summing a split and interleaving take the rest.
-    // The constants were fitted to 600 launches of 32 scans (50^2 to 512^2, 60 to 1130 views, 1 to 12
-    // slices, every choice here); the choice takes 5 % more than the best of a scan's launches in the
-    // geometric mean, 26 % at most, where the timer's step was 10 %.
-    const double geometry = A.mode == SGB_PAR ? 4.4 : (A.mode == SGB_FLAT ? 6.3 : 13.5);
+    // Predicted time in us.  A view of a tile costs each thread its pixels' geometry and taps and the staging
+    // (`scale` us per instruction); CTAs of an SM share its issue slots, one alone taking `alone` times its
+    // share, and a few rounds of them even out less than many.  The pixel-by-pixel kernel waits out each
+    // chunk's copies, the other overlaps them but no chunk takes less.  Summing a split and interleaving slices
+    // take the rest.  Fitted to 5000 launches of 300 scans (48 to 640 pixels a side, 45 to 1200 views, 1 to 16
+    // slices, every form and split): the choice takes 3 % more than the fastest launch of its scan in the
+    // geometric mean.  Every pixel by itself with views split by SMs alone took 20 % more than the choice; on
+    // 17 scans, most of 7 to 15 us, 3 to 10 % less.
+    struct Cost {
+        double par, flat, arc, tap, base, seg, scale, alone, uneven, chunk, split, rank, sum;
+    };
+    static const Cost plain = {3.95, 8.24, 18.4, 2.93, 6.72, 70.9, 0.0013, 2.73, 0.145, 0.81, 1.11, 0.059, 0.702},
+                      slots = {0.094, 0.474, 4.99, 2.53, 14.1, 31.4, 0.00203, 2.71, 0.211, 2.93, 1.66, 0.108, 0.36},
+                      slices = {7.96, 1.83, 7.46, 2.19, 8.73, 38, 0.00206, 2.68, 0.161, 5.3, 2.17, 0.72, 0.25};
     const int sms = std::max(1, num_sms());
     Back2Args best = A;
     double best_us = 1e30;
     for (int form : {B2_FORM_SLOTS, B2_FORM_PLAIN, B2_FORM_FOURS}) {
-        const int ns = form == B2_FORM_SLOTS ? A.sym.ns : 1, sl = form == B2_FORM_FOURS ? 4 : 1;
+        const int ns = form == B2_FORM_SLOTS ? A.sym.ns : 1, sl = form == B2_FORM_FOURS ? 4 : 1, n = ns * sl;
         if (A.want_form != B2_FORM_AUTO && form != A.want_form && !(A.want_form == B2_FORM_FOURS && !fours)) continue;
         if (sl == 4 && (!fours || (A.nslices == 1 && A.want_form != B2_FORM_FOURS))) continue;
+        const Cost &c = n == 1 ? plain : (sl == 4 ? slices : slots);
+        const int ctas = n == 1 ? kB2PlainCtas : kB2Ctas;
         const int hx = ns > 1 ? A.sym.hx : A.nx, hy = ns > 1 ? A.sym.hy : A.ny;
-        const int ctas = ns * sl == 1 ? kB2Ctas<1, 1> : kB2Ctas<4, 1>, seg = ns * sl == 1 ? kB2Seg<1, 1> : kB2Seg<4, 1>;
         const long long groups = floor_div_up(A.nslices, sl);
-        const long long tiles = (long long)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * kB2P) * groups;
-        const double tap = sl == 4 ? 6 : (ns > 1 ? 2.1 : 3.8);
-        const double view = 0.0015 * (kB2P * (geometry + ns * tap) + 10.8 + ns * A.w / 12.0);
+        const double all = (double)floor_div_up(hx, kB2X) * floor_div_up(hy, kB2Y * kB2P) * groups;
+        const long long tiles = std::max(1LL, (long long)std::ceil(all * A.wanted));
+        const double geometry = A.mode == SGB_PAR ? c.par : (A.mode == SGB_FLAT ? c.flat : c.arc);
+        const double view = c.scale * (kB2P * (geometry + ns * c.tap) + c.base + n * A.w / c.seg);
         for (int g = 1; g <= 8 && groups * g <= 65535; g++) {
             if (A.want_split ? g != A.want_split
                              // eight views a rank at least; and the tiles alone may fill the chip
-                             : g > 1 && (A.nv < 8 * g || tiles >= (long long)ctas * sms)) continue;
-            const int busiest = (int)((tiles * g + sms - 1) / sms);
-            const int waves = busiest / ctas, rest = busiest % ctas;
-            const double share = waves * std::max(2.4, (double)ctas) + (rest ? std::max(2.4, (double)rest) : 0);
-            // a chunk of views takes at least its copies' latency
-            const int views = floor_div_up(A.nv, g), vc = std::max(1, std::min({kB2V, seg / 2 / (ns * A.w * 4 * sl), views}));
-            const double us = floor_div_up(views, vc) * std::max(vc * view * share, 0.9 * (waves + (rest ? 1 : 0))) +
-                              (g > 1 ? 1.5 + 0.1 * g + 0.3 * ns * sl * (double)(tiles * g) / sms : 0) +
-                              (sl == 4 ? 3 + 1e-5 * A.nb * (double)A.na * A.nslices : 0);
+                             : g > 1 && (A.nv < 8 * g || tiles >= 2LL * ctas * sms)) continue;
+            const long long busiest = (tiles * g + sms - 1) / sms;
+            const double waves = (double)(busiest / ctas), rest = (double)(busiest % ctas), rounds = waves + (rest > 0);
+            const double share = (waves * std::max(c.alone, (double)ctas) + (rest ? std::max(c.alone, rest) : 0)) *
+                                 (1 + c.uneven / rounds);
+            const int views = floor_div_up(A.nv, g);
+            const int vc = n == 1 ? kB2V : std::max(1, std::min(kB2V, kB2Seg / 2 / (n * A.w * 4)));
+            double us = 0;
+            if (n == 1) {
+                us = views * view * share + floor_div_up(views, vc) * c.chunk * rounds;
+            } else {
+                const int full = views / vc, left = views % vc;
+                us = full * std::max(vc * view * share, c.chunk * rounds) +
+                     (left ? std::max(left * view * share, c.chunk * rounds) : 0);
+            }
+            if (g > 1) us += c.split + c.rank * g + c.sum * n * (double)(tiles * g) / sms;
+            if (sl == 4) us += 8 + 1.2e-5 * A.nb * (double)A.na * A.nslices;
             if (us < best_us) {
                 best_us = us;
                 best.sym.ns = ns;

@@ -142,22 +142,22 @@ struct Back2Args {
     int sl, split;  // slices per CTA (1 or 4) and CTAs that share a tile's views (back2_choose)
     int w, vc;  // staged bins per segment (<= 256; longer ones read global memory) and views per chunk
     ScanSlots sym;
+    float wanted;  // share of the image's tiles that have a pixel inside the mask
     int want_form, want_split;  // the launch asked for: B2_FORM_AUTO and 0 leave the choice to back2_choose
 };
 // Forms of a 2D launch: a pixel at a time; with its images under the scan's symmetry; for four slices.
 enum { B2_FORM_AUTO = -1, B2_FORM_PLAIN = 0, B2_FORM_SLOTS = 1, B2_FORM_FOURS = 2 };
 constexpr int kB2X = 32, kB2Y = 8;  // pixels of a 2D tile that its 256 threads take at a time
 constexpr int kB2P = 4;             // such passes: rows of a tile / 8
-// CTAs that share an SM, by their registers and staged segments
-template <int NS, int SL>
-constexpr int kB2Ctas = NS * SL == 1 ? 5 : 3;
+// CTAs that share an SM, by their registers and staged segments: one pixel at a time, and the others
+constexpr int kB2PlainCtas = 4, kB2Ctas = 3;
 constexpr int kB2V = 32;   // views per chunk, at most
 constexpr int kB2W = 256;  // staged bins per view and slot, at most; the last two stay zero
-// bytes of staged segments, two buffers: kB2Ctas CTAs per SM
-template <int NS, int SL>
-constexpr int kB2Seg = (NS * SL == 1 ? 40 : 64) * 1024;
+constexpr int kB2Seg = 64 * 1024;  // bytes of staged segments, two buffers: kB2Ctas CTAs per SM
+// share of the 2D tiles of an nx x ny mask with a pixel inside it, and how far from the centre such pixels lie
+float back2_wanted(const uint8_t *mask, int nx, int ny, double dx, double dy, double ox, double oy, double *reach);
 // sets w
-void back2_window(Back2Args &A, double dx, double dy);
+void back2_window(Back2Args &A, double dx, double dy, double reach);
 // The launch predicted to be the fastest: with or without the slots, slices one by one or in fours, and
 // the view split.  `fours`: the caller has room for the interleaved slices.
 void back2_choose(Back2Args &A, bool fours);

@@ -74,7 +74,8 @@ def test_fours_and_plain(cuda, kind, image, split, slices):
 
 
 def test_choice_at_larger_sizes(cuda):
-    """320 x 320 from 180 views: images of a pixel for one slice, fours for a stack of eight."""
-    g = dict(kind="par", nb=480, d=1.0, offset=0.0, na=180, orbit=180.0, orbit_start=0.0)
-    plan = S.plan_fbp(C.to_geom(g), S.ImageGeom((320, 320), (1.0, 1.0)))
+    """512 x 512 from 720 views of an arc: images of a pixel for one slice, fours for a stack of eight."""
+    g = dict(kind="arc", nb=788, d=1.0, offset=0.0, na=720, orbit=360.0, orbit_start=0.0, source_offset=0.0, dsd=1200.0,
+             dod=400.0)
+    plan = S.plan_fbp(C.to_geom(g), S.ImageGeom((512, 512), (0.9, 0.9)))
     assert plan.back_form(1)["images"] == 4 and plan.back_form(8)["slices"] == 4
