@@ -296,11 +296,17 @@ SGB_API int sgb_plan_last_timing(sgb_plan *plan, double *ms, int n);
  * info[3] = row pitch of the filtered projections, info[4] = voxels per thread along z,
  * info[5] (when n >= 6) = launches the views are split over, info[6] (when n >= 7) = bytes per
  * stored filtered sample (8: FP32 pairs (y, y[next] - y) or FP16 quads, 4: FP32, 2: BF16),
- * info[7] (when n >= 8) = 1 when the 8-byte samples are FP16 quads (F16 storage). */
+ * info[7] (when n >= 8) = 1 when the 8-byte samples are FP16 quads (F16 storage), info[8] (when n >= 9) =
+ * voxels that share their geometry under the scan's mirror symmetry (1: none), info[9] (when n >= 10) =
+ * thread blocks that share such a tile's views. */
 SGB_API int sgb_plan_info(const sgb_plan *plan, int *info, int n);
 /* Overrides the autotuner's choice of how many launches an FDK plan splits its views over (the
  * later launches add to the volume); 1 <= passes <= min(8, na).  Results agree to rounding. */
 SGB_API int sgb_plan_set_view_passes(sgb_plan *plan, int passes);
+/* FDK plans: 1 takes voxels together with their images under the scan's mirror symmetry, 0 does not; the plan
+ * chooses the one that it predicts to be faster.  SGB_ERR_UNSUPPORTED where the scan has no such symmetry or the
+ * storage form (sgb_plan_info) does not go with it.  Results agree to rounding. */
+SGB_API int sgb_plan_set_mirror(sgb_plan *plan, int mirror);
 /* Launch of a 2D plan's back-projection (no counterpart in the reference).  set_back_form overrides the
  * plan's choice: form 0 takes a pixel at a time, 1 each pixel together with its images under the scan's
  * symmetry (those that have one), 2 four slices at a time, -1 leaves it to the plan; `split` (1..8, 0: the

@@ -329,15 +329,17 @@ int fdk_tma_autotune(sgb_plan *P, cudaStream_t st, bool tune) {
     return SGB_OK;
 }
 
-// The mirrored back-projector, where the scan has a symmetry and its boxes fit.
-int plan_fdk_mirror(sgb_plan *P, const sgb_image_geom *ig, cudaStream_t st) {
+// The mirrored back-projector, where the scan has a symmetry, its boxes fit and it is predicted to be faster
+// than the other (or `always`).
+int plan_fdk_mirror(sgb_plan *P, cudaStream_t st, bool always = false) {
     FdkMirrorArgs &M = P->margs;
-    fdk_mirror_slots(M, P->targs, P->cg.orbit, P->cg.orbit_start, ig->offsets, P->cg.offset_t);
+    fdk_mirror_slots(M, P->targs, P->cg.orbit, P->cg.orbit_start, P->offsets, P->cg.offset_t);
     if (M.nvs * (M.zm ? 2 : 1) == 1) return SGB_OK;
     FdkTmaArgs T = P->targs;  // geometries whose pair boxes are too large keep to plain FP32 boxes
     T.zu = 16;
     SGB_TRY(fdk_tma_prepare(T, P->flags.as<int>(), st));
-    if (fdk_tma_choose(T)) SGB_TRY(fdk_mirror_prepare(M, P->flags.as<int>(), st, &P->mirror));
+    if (fdk_tma_choose(T))
+        SGB_TRY(fdk_mirror_prepare(M, P->flags.as<int>(), st, always ? 1e30 : fdk_tma_predict(T), &P->mirror));
     SGB_CUDA(cudaMemsetAsync(P->flags.p, 0, 4 * sizeof(int), st));
     if (!P->mirror) return SGB_OK;
     M.A.passes = 1;
@@ -403,10 +405,10 @@ int plan_fdk_back(sgb_plan *P, const sgb_image_geom *ig, cudaStream_t st, bool t
     double ry = std::fabs(ig->deltas[1]) * (ig->dims[1] / 2.0 + std::fabs(ig->offsets[1]) + 1);
     P->tma = false;
     if (std::sqrt(rx * rx + ry * ry) < 0.9 * (g.dsd - g.dod)) {
-        if (tune && !A.quad) SGB_TRY(plan_fdk_mirror(P, ig, st));
+        if (tune && !A.quad) SGB_TRY(plan_fdk_mirror(P, st));
         if (!P->mirror) SGB_TRY(fdk_tma_autotune(P, st, tune));
         // quads keep the t grid that the unmirrored form's z-run anchors
-        if (tune && P->tma && A.quad) SGB_TRY(plan_fdk_mirror(P, ig, st));
+        if (tune && P->tma && A.quad) SGB_TRY(plan_fdk_mirror(P, st));
         if (!P->tma && A.elem_bytes == 8) {  // pair or quad boxes too large: plain FP32 boxes
             A.elem_bytes = 4;
             A.quad = 0;
@@ -588,6 +590,23 @@ int sgb_plan_set_view_passes(sgb_plan *P, int passes) {
     return SGB_OK;
 }
 
+int sgb_plan_set_mirror(sgb_plan *P, int mirror) {
+    SGB_REQUIRE(P && P->ct, "plan_set_mirror: needs an FDK plan");
+    cudaStream_t st = 0;
+    if (mirror && !P->mirror) {
+        if (P->tma) SGB_TRY(plan_fdk_mirror(P, st, true));
+        if (!P->mirror) {
+            set_error("plan_set_mirror: the scan has no mirror symmetry that this plan's storage form can use");
+            return SGB_ERR_UNSUPPORTED;
+        }
+    } else if (!mirror && P->mirror) {
+        P->mirror = false;
+        SGB_TRY(fdk_tma_autotune(P, st, true));
+    }
+    SGB_CUDA(cudaStreamSynchronize(st));
+    return SGB_OK;
+}
+
 int sgb_plan_info(const sgb_plan *P, int *info, int n) {
     SGB_REQUIRE(P && info && n >= 5, "plan_info: bad argument");
     info[0] = P->tma ? 1 : 0;
@@ -599,6 +618,8 @@ int sgb_plan_info(const sgb_plan *P, int *info, int n) {
     if (n >= 6) info[5] = A.passes;
     if (n >= 7) info[6] = P->ct ? P->targs.elem_bytes : 4;
     if (n >= 8) info[7] = P->ct ? P->targs.quad : 0;
+    if (n >= 9) info[8] = P->mirror ? P->margs.nvs * (P->margs.zm ? 2 : 1) : 1;
+    if (n >= 10) info[9] = P->mirror ? P->margs.split : 1;
     return SGB_OK;
 }
 

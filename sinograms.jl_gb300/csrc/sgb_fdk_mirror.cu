@@ -104,19 +104,82 @@ size_t fdk_mirror_smem(const FdkMirrorArgs &M, int nstage) {
     return 128 + std::max(ring, part);
 }
 
-int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, bool *fits) {
+namespace {
+
+// Predicted times in us.  A CTA takes for a view its columns' geometry (`column`, arcs `arc` more), `voxel`
+// and per slot `tap` (`tapz` with slots at -z) for each voxel of a run, and `byte` for each byte of its boxes.
+// Taps take up to `two` times as much more where voxels lie several detector rows apart, so that each loads
+// rows of its own, and runs that pass the detector's edge go `edge` times slower.  A second CTA on an SM takes
+// `shared` of the first's time, a few rounds of CTAs even out less than many, a split takes its reduction.
+// Fitted to 3500 launches of 290 FP32 and 1200 of 141 F16 scans (48 to 400 columns a side, 1 to 256 slices, 40
+// to 700 views, voxels 0.1 to 9 detector rows apart, volumes inside the detector and past it): of the two
+// kernels and the mirrored one's runs and splits (powers of two: clusters of others fill the chip worse) the
+// fastest prediction took 4 % more than the fastest launch in the geometric mean, and on 15 scans 4 to 19 %
+// more than the unmirrored kernel; the mirrored kernel wherever its boxes fit had taken up to 3.5 times as much.
+struct FdkCost {
+    double column, arc, voxel, tap, tapz, two, step2, step4, width, slope, byte, shared, uneven, edge, view, sum, rank,
+        fixed;
+};
+constexpr FdkCost kMirrorPair = {0.118, 0.0638, 0.00927, 0.00615, 0.00617, 1.54, 0.125, 0.0227, 0.575, 0.0123,
+                                 8.63e-6, 0.557, 0.0332, 1.93, 0.029, 4.99, 0.151, 10.7};
+constexpr FdkCost kMirrorQuad = {0.106, 0.0663, 0.0144, 0.0102, 0.0243, 0.453, 0.392, 3.19, 1e-3, 0,
+                                 7.86e-6, 0.503, 0.0646, 0.545, 0.01, 5.33, 0, 8.52};
+constexpr FdkCost kPlainPair = {0.0858, 0.122, 0.0145, 0.00734, 0, 0.34, 0.784, 0.784, 1.4e-3, 0.0789,
+                                1e-5, 0.388, 0.0414, 0.111, 0, 0, 0, 9.65};
+constexpr FdkCost kPlainQuad = {0.135, 0.103, 0.00558, 0.00943, 0, 0.0961, 0, 0, 1e9, 0.0078,
+                                1.3e-5, 0.378, 0, 0.101, 0, 0, 0, 10.7};
+
+// Share of the (column, view) pairs of runs of kz voxels from iz0 that pass the detector's first or last row, from
+// a coarse sample of columns and angles.
+double edge_share(const FdkTmaArgs &A, int iz0, int kz, bool whole_runs) {
+    const double limit = (A.nt - 1) / 2.0 - 0.02;
+    double toward[8];
+    for (int a = 0; a < 8; a++) toward[a] = std::cos((a + 0.5) * 0.39269908169872414);  // pi / 8
+    long long out = 0, all = 0;
+    for (int b = 0; iz0 + b * kz < A.nz; b++) {
+        int iz = iz0 + b * kz;
+        if (whole_runs && iz + kz > A.nz && A.nz >= kz) iz = A.nz - kz;
+        const double z = std::max(std::fabs(A.z0 + iz * A.dz), std::fabs(A.z0 + (iz + kz - 1) * A.dz)) * A.inv_dtds;
+        for (int i = 0; i < 36; i++) {
+            const double x = A.x0 + A.dx * (A.nx * (i % 6 + 0.5) / 6 - 0.5), y = A.y0 + A.dy * (A.ny * (i / 6 + 0.5) / 6 - 0.5);
+            const double r = std::hypot(x, y);
+            for (int a = 0; a < 8; a++, all++) out += z * A.dsd_ds > limit * (A.dso_ds - r * toward[a]);
+        }
+    }
+    return all ? (double)out / (double)all : 0;
+}
+
+// A CTA's time per view (slots: voxels per (x, y, z) of the run) and a launch's.
+double cta_view(const FdkCost &c, const FdkTmaArgs &A, int kz, int slots, int nvs, bool zm, double edge) {
+    const double step = std::fabs(A.dz) * A.inv_dtds * A.dsd_ds / A.dso_ds, over = step - (slots == 2 ? c.step2 : c.step4);
+    const double two = 1 + c.two / (1 + std::exp(-std::max(-30.0, std::min(30.0, over / c.width)))) + c.slope * std::max(0.0, over);
+    return (c.column + (A.is_arc ? c.arc * std::sqrt((double)nvs) : 0) + kz * c.voxel + kz * slots * (zm ? c.tapz : c.tap) * two +
+            (double)slots * A.box_bytes * c.byte) *
+           (1 + edge * c.edge);
+}
+double launch_us(const FdkCost &c, double view, int nv, int split, long long ctas, int per) {
+    const long long sms = std::max(1, num_sms()), busiest = (ctas * split + sms - 1) / sms, rounds = (busiest + per - 1) / per;
+    const double t = busiest <= per ? view * (per == 2 ? 1 + c.shared * (busiest - 1) : (double)busiest)
+                                    : view * (1 + c.shared * (per - 1)) * busiest / per * (1 + c.uneven / rounds);
+    return (floor_div_up(nv, split) + c.view * rounds) * t + (split > 1 ? c.sum * rounds + c.rank * split : 0) + c.fixed;
+}
+
+}  // namespace
+
+double fdk_tma_predict(const FdkTmaArgs &A) {
+    const FdkCost &c = A.quad ? kPlainQuad : kPlainPair;
+    const double view = cta_view(c, A, A.zu, 1, 1, false, edge_share(A, 0, A.zu, true));
+    return launch_us(c, view, A.nv, 1, (long long)floor_div_up(A.nx, kTX) * floor_div_up(A.ny, kTY) * floor_div_up(A.nz, A.zu), 2);
+}
+
+int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, double limit_us, bool *fits) {
     *fits = false;
     const int ns = M.nvs * (M.zm ? 2 : 1);
     if (ns == 1) return SGB_OK;
-    const int tx = floor_div_up(M.hx, kTX), ty = floor_div_up(M.hy, kTY), sms = std::max(1, num_sms());
-    // Run length and view split by the time they predict: the busiest SM's CTAs, each so many us per
-    // view.  Fitted to 22 volumes from 51 x 166 x 221 to 512 x 512 x 256: 64 accumulators per thread take
-    // 1.54 us for a CTA alone on its SM and 1.74 us for two (32 accumulators: 1.19 and 1.39), and where
-    // voxels lie 1.5 detector rows or more apart, so that each loads two rows, 2.2 and 2.8 (1.4 and 1.7).
-    // A split costs its reduction, about 4 us, and 1.5% per rank.  The choice came within 10% of the
-    // fastest of all runs and splits on 18 of them, and within 25% on the others.
+    const int tx = floor_div_up(M.hx, kTX), ty = floor_div_up(M.hy, kTY);
+    const FdkCost &c = M.A.quad ? kMirrorQuad : kMirrorPair;
     FdkMirrorArgs best{};
-    double best_us = 1e30;
+    double best_us = limit_us;
     for (int half = 0; half < 2; half++) {
         FdkMirrorArgs T = M;
         FdkTmaArgs &A = T.A;
@@ -140,26 +203,22 @@ int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, bool *fi
         A.box_bytes = (int)(((size_t)A.W * A.H * 8 + 127) / 128 * 128);
         A.nstage = fdk_mirror_smem(T, 4) <= 112 * 1024 ? 4 : 3;
         if (fdk_mirror_smem(T, A.nstage) > 226 * 1024) continue;
-        const int per = fdk_mirror_smem(T, A.nstage) <= 112 * 1024 ? 2 : 1;  // CTAs that fit an SM
-        const bool coarse = std::fabs(A.dz) * A.inv_dtds * A.dsd_ds / A.dso_ds >= 1.5f;
-        const double alone = coarse ? (half ? 1.4 : 2.2) : (half ? 1.19 : 1.54);
-        const double more = coarse ? (half ? 0.3 : 0.6) : 0.20;
+        const double view = cta_view(c, A, T.kz, ns, M.nvs, M.zm, edge_share(A, M.iz0, T.kz, !A.quad));
         const long long ctas = (long long)tx * ty * ntz;
-        for (int g = 1; g <= 8; g++) {
+        for (int g = 1; g <= 8; g *= 2) {
             if (A.nv < 8 * g || ctas * g > (1 << 30) || ntz * g > 65535) break;
-            const long long busiest = (ctas * g + sms - 1) / sms;
-            const double view = busiest <= per ? alone + more * (busiest - 1) : (alone + more * (per - 1)) * busiest / per;
-            const double us = (double)((A.nv + g - 1) / g) * view * (1 + 0.015 * (g - 1)) + (g > 1 ? 4 : 0);
+            T.split = g;
+            const size_t smem = fdk_mirror_smem(T, A.nstage);
+            if (smem > 226 * 1024) break;
+            const double us = launch_us(c, view, A.nv, g, ctas, smem <= 112 * 1024 ? 2 : 1);
             if (us < best_us) {
                 best_us = us;
                 best = T;
-                best.split = g;
+                *fits = true;
             }
         }
     }
-    if (best_us > 1e29) return SGB_OK;
-    M = best;
-    *fits = true;
+    if (*fits) M = best;
     return SGB_OK;
 }
 

@@ -26,9 +26,11 @@ struct FdkMirrorArgs {
 // Slots of a scan's symmetry (nvs and zm; 1 and 0 when it has none that the storage form can use).
 void fdk_mirror_slots(FdkMirrorArgs &M, const FdkTmaArgs &A, double orbit, double orbit_start, const double *offsets,
                       double offset_t);
-// Run length, box (device pre-pass) and ring; false when the mirrored boxes do not fit shared memory
-// or the volume is too small for it.
-int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, bool *fits);
+// Predicted time in us of the unmirrored kernel, prepared with its run length and box.
+double fdk_tma_predict(const FdkTmaArgs &A);
+// Run length, view split, box (device pre-pass) and ring; false when the mirrored boxes do not fit shared memory
+// or no launch is predicted to take less than limit_us.
+int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, double limit_us, bool *fits);
 int launch_fdk_mirror(const FdkMirrorArgs &M, const CUtensorMap &map, cudaStream_t st);
 size_t fdk_mirror_smem(const FdkMirrorArgs &M, int nstage);
 // one storage form and detector each (sgb_fdk_mirror_<form>_<detector>.cu)

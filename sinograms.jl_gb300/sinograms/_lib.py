@@ -109,6 +109,7 @@ _SIGS = {
     "sgb_plan_info": (c_int, [P, P, c_int]),
     "sgb_plan_sync": (c_int, [P, P]),
     "sgb_plan_set_view_passes": (c_int, [P, c_int]),
+    "sgb_plan_set_mirror": (c_int, [P, c_int]),
     "sgb_plan_set_back_form": (c_int, [P, c_int, c_int]),
     "sgb_plan_back_form": (c_int, [P, c_int, P, c_int]),
     "sgb_measure_peaks": (c_int, [P, c_int, P]),

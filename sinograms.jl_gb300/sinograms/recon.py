@@ -76,10 +76,10 @@ class _Plan:
 
     def info(self) -> dict:
         """Execution layout: TMA-staged FDK kernel in use, staged box, row pitch, z-unroll."""
-        a = np.zeros(8, dtype=np.int32)
-        _status(_lib.lib().sgb_plan_info(self._h, ptr(a), 8), "plan_info")
+        a = np.zeros(10, dtype=np.int32)
+        _status(_lib.lib().sgb_plan_info(self._h, ptr(a), 10), "plan_info")
         return dict(tma=bool(a[0]), box=(int(a[1]), int(a[2])), pitch=int(a[3]), zu=int(a[4]), view_passes=int(a[5]),
-                    sample_bytes=int(a[6]), f16_quads=bool(a[7]))
+                    sample_bytes=int(a[6]), f16_quads=bool(a[7]), images=int(a[8]), view_split=int(a[9]))
 
     def set_view_passes(self, passes: int):
         """FDK plans: split the views over `passes` launches (overrides the autotuner's choice)."""
@@ -123,6 +123,11 @@ class FDKplan(_Plan):
     @property
     def view_weight(self):
         return fdk_view_weight(self.rg)
+
+    def set_mirror(self, mirror: bool):
+        """Take voxels together with their images under the scan's mirror symmetry, or not (overrides the
+        plan's choice; an error where the scan has none that the storage form can use)."""
+        _status(_lib.lib().sgb_plan_set_mirror(self._h, int(bool(mirror))), "plan_set_mirror")
 
 
 def plan_fbp(rg, ig: ImageGeom, window: Window = Window(), npad: int | None = None, decon1: bool = True,

@@ -21,6 +21,7 @@ def test_repeated_calls_agree(cuda, kind, storage, na):
     ig = dict(dims=(48, 44, 20), deltas=(0.75, 0.75, 0.75), offsets=(0.0, 0.0, 0.0))
     proj = O.ellipsoid_proj(g, C.ELL3).astype(np.float32)
     plan = S.plan_fbp(C.to_geom(g), C.to_image(ig), storage=storage)
+    plan.set_mirror(True)
     first = S.fdk(plan, proj)
     assert O.rel_rmse(first, O.fdk(g, ig, proj)) < C.form_bars(storage, na)[0]
     for _ in range(30):
