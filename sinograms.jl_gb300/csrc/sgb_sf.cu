@@ -37,7 +37,9 @@
 //     have the same elements in the views that see them alike, at the same bins or at those mirrored about
 //     the detector's centre.  So the forward kernel sums a view's bins over the image together with the
 //     bins of the views that are its images, over the image's images, and the back-projector takes a pixel
-//     with its images: each element is evaluated once for two or four.  Mirrored elements agree to rounding
+//     with its images: each element is evaluated once for two or four.  (Over half a turn of parallel beams
+//     the images of a view are half as many as those of a pixel.)  Scans without symmetry have a forward
+//     kernel of their own, sf_project_plain_kernel.  Mirrored elements agree to rounding
 //     only (wb + K a and wb - K a round differently): both evaluate them at the forward sweep's view.
 // Both directions are bound by issue, most of it the elements.  888 x 90 arc, 512^2: forward 437 -> 136 us,
 // back 242 -> 115 us with four slots against one element at a time; a pair of calls 683 -> 264 us.
@@ -46,6 +48,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "sgb_common.cuh"
@@ -93,6 +96,7 @@ struct SfArgs {
     int gsplit;  // back: CTAs of a cluster that share a tile's items
     int nitem;   // back: items
     int nrep;    // forward: views that are not images of others
+    int fslots;  // forward: slots that give other views (half a turn of parallel beams: half of them)
     ScanSlots sym;
     float wb, ax, ay, axy, hx, hy;
 };
@@ -337,6 +341,99 @@ __global__ void sf_image_kernel(const float *__restrict__ image, const uint8_t *
     }
 }
 
+// The record of a staged pixel (parallel beams: the view's own but for uc).
+template <int GEO>
+__device__ __forceinline__ SfRec sf_staged(const SfView &V, float4 a0, const float4 *a1) {
+    SfRec r;
+    r.uc = a0.x;
+    if (GEO == 0) {
+        r.d0 = V.p0;
+        r.d1 = V.p1;
+        r.d2 = V.p2;
+        r.d3 = V.p3;
+        r.hr01 = V.phr01;
+        r.hr23 = V.phr23;
+        r.c3 = V.pc3;
+    } else {
+        r.d0 = a0.y;
+        r.d1 = a0.z;
+        r.d2 = a0.w;
+        r.d3 = a1->x;
+        r.hr01 = a1->y;
+        r.hr23 = a1->z;
+        r.c3 = a1->w;
+    }
+    return r;
+}
+
+// One view at a time, for scans without symmetry: a line's pixels are staged and summed, one barrier between, and
+// the CTAs of an SM hide each other's loads.  With one sum per element and bin, fetching a line ahead as the kernel
+// below does costs more than it hides (arc, 257 x 257, 384 bins x 181 views: 235 us, a line ahead 256).
+template <int GEO>
+__global__ void __launch_bounds__(kFwdThreads) sf_project_plain_kernel(SfArgs A, const SfView *__restrict__ views,
+                                                                       const float2 *__restrict__ rays,
+                                                                       const float *__restrict__ xcs,
+                                                                       const float *__restrict__ ycs,
+                                                                       const float *__restrict__ image,
+                                                                       const float *__restrict__ imaget,
+                                                                       float *__restrict__ sino) {
+    constexpr int CAP = kFwdCap<1>;
+    __shared__ float4 s0[2][CAP];                // uc, d0, d1, d2
+    __shared__ float4 s1[GEO != 0 ? 2 : 1][CAP];  // d3, hr01, hr23, c3 (fan beams)
+    __shared__ float2 s2[2][CAP];                // h, pixel value
+    const int v = blockIdx.y, tid = threadIdx.x;
+    const int k0 = blockIdx.x * kFwdBins, kend = min(k0 + kFwdBins, A.nb);
+    const int ka = k0 + kFwdBpt * tid, kb = min(ka + kFwdBpt, A.nb);  // this thread's bins [ka, kb)
+    const SfView V = views[v];
+    const bool rows = V.rows != 0;
+    const int nal = rows ? A.nx : A.ny, nln = rows ? A.ny : A.nx;
+    const float *lcs = rows ? ycs : xcs, *src = rows ? image : imaget;
+    const float hl = rows ? A.hy : A.hx;
+    const float2 *R = rays + (size_t)v * (A.nb + 1);
+    const float2 cl = R[k0], ch = R[kend];
+    const bool active = ka < A.nb;
+    const float2 bl = R[min(ka, A.nb)], bh = R[max(kb, 0)];
+    const float e0 = sf_bound<GEO>(ka, A), e1 = sf_bound<GEO>(ka + 1, A), e2 = sf_bound<GEO>(ka + 2, A);
+    const int per = (nln + A.splits - 1) / A.splits, jb = blockIdx.z * per, je = min(nln, jb + per);
+    float acc0 = 0.f, acc1 = 0.f;
+    int buf = 0;
+    for (int j = jb; j < je; j++) {
+        const float lc = lcs[j], L0 = lc - hl, L1 = lc + hl;
+        int ia, ib;
+        sf_range(cl, ch, L0, L1, nal, ia, ib);
+        if (ia > ib) continue;  // same for the whole CTA
+        int qa = 0, qb = -1;
+        if (active) sf_range(bl, bh, L0, L1, nal, qa, qb);
+        for (int p0 = ia; p0 <= ib; p0 += CAP) {
+            const int p1 = min(ib, p0 + CAP - 1);
+            for (int t = tid; t <= p1 - p0; t += kFwdThreads) {
+                const int i = p0 + t;
+                const float val = __ldg(src + (size_t)nal * j + i);
+                const SfRec r = sf_pixel<GEO>(V, A, __ldg(xcs + (rows ? i : j)), __ldg(ycs + (rows ? j : i)));
+                s0[buf][t] = make_float4(r.uc, r.d0, r.d1, r.d2);
+                if (GEO != 0) s1[buf][t] = make_float4(r.d3, r.hr01, r.hr23, r.c3);
+                s2[buf][t] = make_float2(r.h, val);
+            }
+            __syncthreads();
+            const int ta = max(qa, p0), tb = min(qb, p1);
+            for (int i = ta; i <= tb; i++) {
+                const int t = i - p0;
+                const float2 a2 = s2[buf][t];
+                const SfRec r = sf_staged<GEO>(V, s0[buf][t], GEO != 0 ? &s1[buf][t] : nullptr);
+                const float g0 = sf_cdf<GEO>(__fsub_rn(e0, r.uc), r), g1 = sf_cdf<GEO>(__fsub_rn(e1, r.uc), r);
+                const float g2 = sf_cdf<GEO>(__fsub_rn(e2, r.uc), r);
+                acc0 = __fmaf_rn(__fmul_rn(a2.x, __fsub_rn(g1, g0)), a2.y, acc0);
+                acc1 = __fmaf_rn(__fmul_rn(a2.x, __fsub_rn(g2, g1)), a2.y, acc1);
+            }
+            buf ^= 1;
+        }
+    }
+    // splits > 1: partial sums, added in split order by sf_sum_splits
+    float *row = sino + (size_t)A.nb * (v + (size_t)A.na * blockIdx.z);
+    if (active) row[ka] = acc0;
+    if (ka + 1 < A.nb) row[ka + 1] = acc1;
+}
+
 template <int GEO, int NS>
 __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const SfView *__restrict__ views,
                                                                  const float2 *__restrict__ rays,
@@ -446,28 +543,8 @@ __global__ void __launch_bounds__(kFwdThreads) sf_project_kernel(SfArgs A, const
         const int ta = max(cur.qa, cur.p0), tb = min(cur.qb, cur.p1);
         for (int i = ta; i <= tb; i++) {
             const int t = i - cur.p0;
-            const float4 a0 = s0[buf][t];
             const float h = s2[buf][t];
-            SfRec r;
-            r.uc = a0.x;
-            if (GEO == 0) {
-                r.d0 = V.p0;
-                r.d1 = V.p1;
-                r.d2 = V.p2;
-                r.d3 = V.p3;
-                r.hr01 = V.phr01;
-                r.hr23 = V.phr23;
-                r.c3 = V.pc3;
-            } else {
-                const float4 a1 = s1[buf][t];
-                r.d0 = a0.y;
-                r.d1 = a0.z;
-                r.d2 = a0.w;
-                r.d3 = a1.x;
-                r.hr01 = a1.y;
-                r.hr23 = a1.z;
-                r.c3 = a1.w;
-            }
+            const SfRec r = sf_staged<GEO>(V, s0[buf][t], GEO != 0 ? &s1[buf][t] : nullptr);
             const float g0 = sf_cdf<GEO>(__fsub_rn(e0, r.uc), r), g1 = sf_cdf<GEO>(__fsub_rn(e1, r.uc), r);
             const float g2 = sf_cdf<GEO>(__fsub_rn(e2, r.uc), r);
             const float w0 = __fmul_rn(h, __fsub_rn(g1, g0)), w1 = __fmul_rn(h, __fsub_rn(g2, g1));
@@ -646,12 +723,16 @@ int sf_launch_forward(int kind, const SfArgs &A, const SfView *views, const floa
                       const float *ycs, const float *src, const float *srct, const int4 *reps, float *dst,
                       cudaStream_t st) {
     const dim3 grid((A.nb + kFwdBins - 1) / kFwdBins, A.nrep, A.splits);
-    if (kind == SGB_PAR)
-        sf_project_kernel<0, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
-    else if (kind == SGB_ARC)
-        sf_project_kernel<1, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
-    else
-        sf_project_kernel<2, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
+    auto go = [&](auto geo) {
+        constexpr int GEO = decltype(geo)::value;
+        if constexpr (NS == 1)
+            sf_project_plain_kernel<GEO><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, dst);
+        else
+            sf_project_kernel<GEO, NS><<<grid, kFwdThreads, 0, st>>>(A, views, rays, xcs, ycs, src, srct, reps, dst);
+    };
+    if (kind == SGB_PAR) go(std::integral_constant<int, 0>{});
+    else if (kind == SGB_ARC) go(std::integral_constant<int, 1>{});
+    else go(std::integral_constant<int, 2>{});
     return after_launch("sf_project_kernel");
 }
 
@@ -790,16 +871,17 @@ void sf_items(const ScanSlots &S, int na, bool half, std::vector<int4> &reps, st
 }
 
 // Line splits of the forward projector: enough CTAs for about two resident waves of four-warp
-// CTAs (16 per SM), at most 32 and at least 8 image lines per CTA.
-int sf_default_splits(const SfGeo &G, int nrep) {
+// CTAs (16 per SM), at most 32 and at least 8 image lines per CTA (4 without shared elements: 64 x 64 pixels,
+// 100 bins x 61 views 16.7 and 15.0 us).
+int sf_default_splits(const SfGeo &G, int nrep, int ns) {
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
     const long long ctas = (long long)((G.nb + kFwdBins - 1) / kFwdBins) * nrep;
     const long long want = 2LL * 16 * std::max(sms, 1);
     int s = (int)std::min<long long>(32, std::max<long long>(1, (want + ctas - 1) / ctas));
-    const int lines = std::max(G.nx, G.ny);
-    while (s > 1 && lines / s < 8) s--;
+    const int lines = std::max(G.nx, G.ny), least = ns == 1 ? 4 : 8;
+    while (s > 1 && lines / s < least) s--;
     return s;
 }
 
@@ -828,8 +910,8 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
         sf_image_kernel<<<dim3((G.nx + 31) / 32, (G.ny + 31) / 32), dim3(32, 8), 0, st>>>(
             src, P->mask_dev, G.nx, G.ny, P->img.as<float>(), P->img.as<float>() + nimg);
         SGB_TRY(after_launch("sf_image_kernel"));
-        auto go = P->A.sym.ns == 4 ? sf_launch_forward<4>
-                                   : (P->A.sym.ns == 2 ? sf_launch_forward<2> : sf_launch_forward<1>);
+        auto go = P->A.fslots == 4 ? sf_launch_forward<4>
+                                   : (P->A.fslots == 2 ? sf_launch_forward<2> : sf_launch_forward<1>);
         SGB_TRY(go(G.kind, P->A, views, P->rays.as<float2>(), xcs, ycs, P->img.as<float>(), P->img.as<float>() + nimg,
                    P->reps.as<int4>(), dst, st));
         if (splits > 1) {
@@ -897,6 +979,11 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
     const bool centred = 2 * G.wb == G.nb - 1.0;
     sf_items(A.sym, G.na, G.kind == SGB_PAR && centred && G.ox == 0 && G.oy == 0, reps, items);
     A.nrep = (int)reps.size();
+    A.fslots = 1;
+    for (const int4 &e : reps) {
+        if (A.sym.ns == 4 && !(e.z & e.w & kSfDup)) A.fslots = 4;
+        else if (A.sym.ns > 1 && !(e.y & kSfDup)) A.fslots = std::max(A.fslots, 2);
+    }
     A.nitem = (int)items.size();
     DevBuf items_dev;
     SGB_TRY(P->reps.reserve(sizeof(int4) * reps.size()));
@@ -907,7 +994,7 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
     SGB_TRY(P->item_rows.reserve(sizeof(int4) * items.size()));
     SGB_TRY(P->zeros.reserve(sizeof(float) * G.nb));
     SGB_CUDA(cudaMemsetAsync(P->zeros.p, 0, sizeof(float) * G.nb, st));
-    A.splits = sf_default_splits(G, A.nrep);
+    A.splits = sf_default_splits(G, A.nrep, A.fslots);
     // back: about four CTAs of 256 pixels per SM, at least 8 views each
     const long long tiles = (long long)((A.sym.hx + kBackTx - 1) / kBackTx) * ((A.sym.hy + kBackTy - 1) / kBackTy);
     A.gsplit = (int)std::max<long long>(1, std::min<long long>({8, G.na / 8, (4LL * std::max(1, num_sms()) + tiles / 2) / tiles}));
