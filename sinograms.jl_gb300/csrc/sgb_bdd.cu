@@ -836,9 +836,9 @@ bool back_fits(const BddArgs &G) {
     return 16 * (size_t)((G.nDet + 1 + 7) / 8 * 8) + 8 * (size_t)kWarps * (G.nPix + G.nPix / 16 + 1) <= 220 * 1024;
 }
 // A mapped bin's width in pixels at the image centre; up to kDirectStep the direct kernel projects.
-// 90 views, us a projection, prefix and direct: 512^2, bins of 0.6 pixels 145 and 112, 1.0 131 and
-// 134, 2.0 120 and 107, 6.0 110 and 87; 1024^2, 0.6 494 and 312, 6.0 300 and 210; 256^2, 79 and 67,
-// 70 and 62.  Wider bins keep the prefix form: its differences stay good to FP32 however many pixels
+// us a projection, prefix and direct, 512^2 from 90 views: bins of 0.6 pixels 143 and 107, 1.0 110 and 113,
+// 1.2 101 and 96, 2.0 89 and 78, 4.0 78 and 62; from 360 views 538 and 303, 411 and 335, 380 and 305, 335 and
+// 249, 290 and 194.  Wider bins keep the prefix form: its differences stay good to FP32 however many pixels
 // lie in a bin.
 constexpr double kDirectStep = 6.0;
 double central_step(const BddArgs &G) { return G.dSize * G.DS0 / (G.DSD * G.pSize); }
@@ -854,8 +854,9 @@ int split_items(int n, long long base, int res) {
     const long long sms = std::max(1, num_sms()), wave = sms * res;
     int best = n;
     double tb = 1e300;
-    for (int s = 1; s <= n; s++) {
+    for (int s = 1; s <= n;) {
         const int per = (n + s - 1) / s;
+        s = per > 1 ? (n + per - 2) / (per - 1) : n + 1;  // the next s with another per
         const long long ctas = base * ((n + per - 1) / per), rest = ctas % wave;
         const double last = rest ? std::max(0.7 * res, (double)((rest + sms - 1) / sms)) : 0.0;
         const double t = ((double)(ctas / wave) * res + last) * (per + 1);
