@@ -271,12 +271,14 @@ SGB_API int sgb_plan_filter(const sgb_plan *plan, double *Hk, int *npad);
 /* fdk(plan, proj), src/fbp3/fdk.jl:65-81: proj (ns,nt,na) -> image (nx,ny,nz). */
 SGB_API int sgb_fdk(sgb_plan *plan, const float *proj, float *image, int flags, void *stream);
 /* fbp(plan, sino) for one 2D sinogram or a stack, src/fbp2/fbp.jl:24-68:
- * sino (nb, na, nslices) -> image (nx, ny, nslices). */
+ * sino (nb, na, nslices) -> image (nx, ny, nslices).  The filtered rows stay in the plan: calls on one
+ * plan are serialised on one stream. */
 SGB_API int sgb_fbp(sgb_plan *plan, const float *sino, float *image, int nslices, int flags,
             void *stream);
 /* The two stages of fbp(plan, sino) (fbp.jl:72-86) for a 2D plan: view weights + ramp
  * filter (fbp_sino_filter), and the plan's back-projector (fbp_back) on filtered rows.
- * Shapes as sgb_fbp; filtered is (nb, na, nslices). */
+ * Shapes as sgb_fbp; filtered is (nb, na, nslices).  sgb_fbp_backproject with device pointers keeps nothing of
+ * a call in the plan: such calls may run on several streams and threads at a time, and in CUDA graphs. */
 SGB_API int sgb_fbp_filter_rows(sgb_plan *plan, const float *sino, float *filtered, int nslices,
                                 int flags, void *stream);
 SGB_API int sgb_fbp_backproject(sgb_plan *plan, const float *filtered, float *image, int nslices,

@@ -42,7 +42,7 @@
 //     kernel of their own, sf_project_plain_kernel.  Mirrored elements agree to rounding
 //     only (wb + K a and wb - K a round differently): both evaluate them at the forward sweep's view.
 // Both directions are bound by issue, most of it the elements.  888 x 90 arc, 512^2: forward 437 -> 136 us,
-// back 242 -> 115 us with four slots against one element at a time; a pair of calls 683 -> 264 us.
+// back 260 -> 115 us with four slots against one element at a time; a pair of calls 683 -> 262 us.
 // Plans compute the per-view constants and the boundary-ray table once, in FP64 on the device.
 #include <cooperative_groups.h>
 #include <algorithm>
