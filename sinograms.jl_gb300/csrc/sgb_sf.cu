@@ -47,6 +47,7 @@
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <memory>
 #include <type_traits>
 #include <vector>
@@ -240,10 +241,8 @@ __device__ __forceinline__ void sf_range(float2 lo, float2 hi, float L0, float L
 }
 
 // ------------------------------------------------------------------- set-up (FP64)
-__global__ void sf_setup_views(SfGeo G, const double *betas, SfView *views) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= G.na) return;
-    const double b = betas[v], cb = cos(b), sb = sin(b);
+__device__ SfView sf_view_at(const SfGeo &G, double b) {
+    const double cb = cos(b), sb = sin(b);
     const double hx = 0.5 * fabs(G.dx), hy = 0.5 * fabs(G.dy);
     SfView V{};
     V.cb = (float)cb;
@@ -276,7 +275,18 @@ __global__ void sf_setup_views(SfGeo G, const double *betas, SfView *views) {
         const bool rows_ok = ys < G.ylo || ys > G.yhi, cols_ok = xs < G.xlo || xs > G.xhi;
         V.rows = pref_rows ? (rows_ok || !cols_ok) : !(cols_ok || !rows_ok);
     }
-    views[v] = V;
+    return V;
+}
+
+// The constants of `nview` views, and of the back-projector's items (their view and map).
+__global__ void sf_setup_views(SfGeo G, const double *betas, int nview, SfView *views, int nitem, const int2 *items,
+                               SfView *item_views) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nview) views[i] = sf_view_at(G, betas[i]);
+    if (i >= nitem) return;
+    SfView V = sf_view_at(G, betas[items[i].x]);
+    V.map = items[i].y;
+    item_views[i] = V;
 }
 
 // Boundary rays: for boundary j (u = j - 1/2, j = 0..nb) the along-coordinate of its crossing with
@@ -579,15 +589,6 @@ __global__ void sf_sum_splits(const float *__restrict__ part, int splits, long l
 }
 
 // ------------------------------------------------------------------- back
-// The items' view constants, in order.
-__global__ void sf_item_views(const SfItem *items, int n, const SfView *views, SfView *out, int4 *rows) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = views[items[i].rep];
-    out[i].map = items[i].map;
-    rows[i] = items[i].rows;
-}
-
 template <int GEO, int NS>
 __global__ void __launch_bounds__(kBackTx *kBackTy) sf_back_kernel(SfArgs A, const SfView *__restrict__ views,
                                                                    const float *__restrict__ xcs,
@@ -747,10 +748,17 @@ using namespace sgb;
 struct sgb_sf_plan {
     SfGeo G{};
     SfArgs A{};
-    DevBuf betas, views, rays, axes, mask, din, dout, part, img;
-    DevBuf reps;  // forward: the representative views' images
-    DevBuf item_views, item_rows, zeros;  // back: the items' constants and rows; a row of zeros
+    DevBuf block, din, dout, part;
+    // in the block; views, rays, reps and img are the forward projector's, the items and zeros the other's
+    const float *axes = nullptr;
     const uint8_t *mask_dev = nullptr;
+    const SfView *views = nullptr;
+    const float2 *rays = nullptr;
+    const int4 *reps = nullptr;  // the representative views' images
+    float *img = nullptr;        // the masked image and its transpose
+    const SfView *item_views = nullptr;
+    const int4 *item_rows = nullptr;
+    const float *zeros = nullptr;  // a row
 };
 
 namespace {
@@ -871,16 +879,16 @@ void sf_items(const ScanSlots &S, int na, bool half, std::vector<int4> &reps, st
 }
 
 // Line splits of the forward projector: enough CTAs for about two resident waves of four-warp
-// CTAs (16 per SM), at most 32 and at least 8 image lines per CTA (4 without shared elements: 64 x 64 pixels,
-// 100 bins x 61 views 16.7 and 15.0 us).
-int sf_default_splits(const SfGeo &G, int nrep, int ns) {
+// CTAs (16 per SM), at most 32 and at least 8 image lines per CTA (4 in a plan without shared elements: 64 x 64
+// pixels, 100 bins x 61 views 16.7 and 15.0 us; a one-shot call allocates the partial rows, which costs more).
+int sf_default_splits(const SfGeo &G, int nrep, int ns, bool kept) {
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
     const long long ctas = (long long)((G.nb + kFwdBins - 1) / kFwdBins) * nrep;
     const long long want = 2LL * 16 * std::max(sms, 1);
     int s = (int)std::min<long long>(32, std::max<long long>(1, (want + ctas - 1) / ctas));
-    const int lines = std::max(G.nx, G.ny), least = ns == 1 ? 4 : 8;
+    const int lines = std::max(G.nx, G.ny), least = ns == 1 && kept ? 4 : 8;
     while (s > 1 && lines / s < least) s--;
     return s;
 }
@@ -896,8 +904,7 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
         SGB_TRY(P->dout.reserve(nout * sizeof(float)));
         out_dev = P->dout.as<float>();
     }
-    const float *xcs = P->axes.as<float>(), *ycs = xcs + G.nx;
-    const SfView *views = P->views.as<SfView>();
+    const float *xcs = P->axes, *ycs = xcs + G.nx;
     const float *src = static_cast<const float *>(in_dev);
     if (forward) {
         const int splits = P->A.splits;
@@ -908,12 +915,11 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
             dst = P->part.as<float>();
         }
         sf_image_kernel<<<dim3((G.nx + 31) / 32, (G.ny + 31) / 32), dim3(32, 8), 0, st>>>(
-            src, P->mask_dev, G.nx, G.ny, P->img.as<float>(), P->img.as<float>() + nimg);
+            src, P->mask_dev, G.nx, G.ny, P->img, P->img + nimg);
         SGB_TRY(after_launch("sf_image_kernel"));
         auto go = P->A.fslots == 4 ? sf_launch_forward<4>
                                    : (P->A.fslots == 2 ? sf_launch_forward<2> : sf_launch_forward<1>);
-        SGB_TRY(go(G.kind, P->A, views, P->rays.as<float2>(), xcs, ycs, P->img.as<float>(), P->img.as<float>() + nimg,
-                   P->reps.as<int4>(), dst, st));
+        SGB_TRY(go(G.kind, P->A, P->views, P->rays, xcs, ycs, P->img, P->img + nimg, P->reps, dst, st));
         if (splits > 1) {
             sf_sum_splits<<<(unsigned)((nsino + 255) / 256), 256, 0, st>>>(dst, splits, (long long)nsino, out_dev);
             SGB_TRY(after_launch("sf_sum_splits"));
@@ -921,8 +927,7 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
     } else {
         auto go = P->A.sym.ns == 4 ? sf_launch_back_kind<4>
                                    : (P->A.sym.ns == 2 ? sf_launch_back_kind<2> : sf_launch_back_kind<1>);
-        SGB_TRY(go(G.kind, P->A, P->item_views.as<SfView>(), xcs, ycs, src, P->mask_dev, P->item_rows.as<int4>(),
-                   P->zeros.as<float>(), out_dev, st));
+        SGB_TRY(go(G.kind, P->A, P->item_views, xcs, ycs, src, P->mask_dev, P->item_rows, P->zeros, out_dev, st));
     }
     if (!(flags & SGB_DEVICE_PTRS))
         SGB_CUDA(cudaMemcpyAsync(out, out_dev, nout * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -931,36 +936,14 @@ int sf_run(sgb_sf_plan *P, bool forward, const float *in, float *out, int flags,
     return SGB_OK;
 }
 
-}  // namespace
+// What a plan is for.
+enum { SF_FORWARD = 1, SF_BACK = 2 };
 
-extern "C" {
-
-int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf_plan **out) {
-    SGB_REQUIRE(out, "sf_plan_create: null argument");
-    *out = nullptr;
+int sf_plan(const sgb_sino_geom *rg, const sgb_image_geom *ig, int uses, std::unique_ptr<sgb_sf_plan> &out) {
     auto P = std::make_unique<sgb_sf_plan>();
     SGB_TRY(sf_geometry(rg, ig, &P->G));
     SfGeo &G = P->G;
     cudaStream_t st = nullptr;
-    const std::vector<double> betas = view_angles(rg->na, rg->orbit, rg->orbit_start);
-    SGB_TRY(P->betas.reserve(sizeof(double) * G.na));
-    SGB_CUDA(cudaMemcpyAsync(P->betas.p, betas.data(), sizeof(double) * G.na, cudaMemcpyHostToDevice, st));
-    std::vector<float> axes(G.nx + G.ny);
-    for (int i = 0; i < G.nx; i++) axes[i] = (float)(G.dx * (i - ((G.nx - 1) / 2.0 + G.ox)));
-    for (int j = 0; j < G.ny; j++) axes[G.nx + j] = (float)(G.dy * (j - ((G.ny - 1) / 2.0 + G.oy)));
-    SGB_TRY(P->axes.reserve(sizeof(float) * axes.size()));
-    SGB_CUDA(cudaMemcpyAsync(P->axes.p, axes.data(), sizeof(float) * axes.size(), cudaMemcpyHostToDevice, st));
-    if (ig->mask) {
-        const size_t n = (size_t)G.nx * G.ny;
-        bool all = true;
-        for (size_t i = 0; i < n && all; i++) all = ig->mask[i] != 0;
-        if (!all) {
-            SGB_TRY(P->mask.reserve(n));
-            SGB_CUDA(cudaMemcpyAsync(P->mask.p, ig->mask, n, cudaMemcpyHostToDevice, st));
-            P->mask_dev = P->mask.as<uint8_t>();
-        }
-    }
-    SGB_TRY(P->img.reserve(sizeof(float) * 2 * (size_t)G.nx * G.ny));  // here: a call may be captured
     SfArgs &A = P->A;
     A.nb = G.nb;
     A.na = G.na;
@@ -985,31 +968,87 @@ int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf
         else if (A.sym.ns > 1 && !(e.y & kSfDup)) A.fslots = std::max(A.fslots, 2);
     }
     A.nitem = (int)items.size();
-    DevBuf items_dev;
-    SGB_TRY(P->reps.reserve(sizeof(int4) * reps.size()));
-    SGB_CUDA(cudaMemcpyAsync(P->reps.p, reps.data(), sizeof(int4) * reps.size(), cudaMemcpyHostToDevice, st));
-    SGB_TRY(items_dev.reserve(sizeof(SfItem) * items.size()));
-    SGB_CUDA(cudaMemcpyAsync(items_dev.p, items.data(), sizeof(SfItem) * items.size(), cudaMemcpyHostToDevice, st));
-    SGB_TRY(P->item_views.reserve(sizeof(SfView) * items.size()));
-    SGB_TRY(P->item_rows.reserve(sizeof(int4) * items.size()));
-    SGB_TRY(P->zeros.reserve(sizeof(float) * G.nb));
-    SGB_CUDA(cudaMemsetAsync(P->zeros.p, 0, sizeof(float) * G.nb, st));
-    A.splits = sf_default_splits(G, A.nrep, A.fslots);
+    // The tables are one block, its first part one copy; a one-shot call pays for no more than it reads.
+    const bool fwd = uses & SF_FORWARD;
+    if (!fwd) reps.clear();
+    if (!(uses & SF_BACK)) items.clear();
+    std::vector<char> host;
+    size_t bytes = 0;
+    auto place = [&bytes](size_t n) {
+        const size_t at = bytes;
+        bytes = (bytes + n + 255) / 256 * 256;
+        return at;
+    };
+    auto put = [&](const void *p, size_t n) {
+        const size_t at = place(n);
+        host.resize(bytes);
+        if (n) std::memcpy(host.data() + at, p, n);
+        return at;
+    };
+    const std::vector<double> betas = view_angles(rg->na, rg->orbit, rg->orbit_start);
+    const size_t betas_at = put(betas.data(), sizeof(double) * G.na);
+    std::vector<float> row(G.nx + G.ny);
+    for (int i = 0; i < G.nx; i++) row[i] = (float)(G.dx * (i - ((G.nx - 1) / 2.0 + G.ox)));
+    for (int j = 0; j < G.ny; j++) row[G.nx + j] = (float)(G.dy * (j - ((G.ny - 1) / 2.0 + G.oy)));
+    const size_t axes_at = put(row.data(), sizeof(float) * row.size());
+    const size_t nimg = (size_t)G.nx * G.ny;
+    const bool masked = ig->mask && std::memchr(ig->mask, 0, nimg);
+    const size_t mask_at = masked ? put(ig->mask, nimg) : 0;
+    const size_t reps_at = put(reps.data(), sizeof(int4) * reps.size());
+    std::vector<int4> rows;
+    std::vector<int2> maps;
+    for (const SfItem &it : items) {
+        rows.push_back(it.rows);
+        maps.push_back(make_int2(it.rep, it.map));
+    }
+    const size_t rows_at = put(rows.data(), sizeof(int4) * rows.size()), maps_at = put(maps.data(), sizeof(int2) * maps.size());
+    row.assign(G.nb, 0.f);
+    const size_t zeros_at = put(row.data(), sizeof(float) * G.nb);
+    const long long nray = fwd ? (long long)G.na * (G.nb + 1) : 0;
+    const size_t views_at = place(sizeof(SfView) * G.na), item_views_at = place(sizeof(SfView) * items.size());
+    const size_t rays_at = place(sizeof(float2) * (size_t)nray);
+    const size_t img_at = place(fwd ? 2 * sizeof(float) * nimg : 0);  // here: a call may be captured
+    SGB_TRY(P->block.reserve(bytes));
+    char *base = P->block.as<char>();
+    SGB_CUDA(cudaMemcpyAsync(base, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+    const double *betas_dev = reinterpret_cast<double *>(base + betas_at);
+    SfView *views = reinterpret_cast<SfView *>(base + views_at), *item_views = reinterpret_cast<SfView *>(base + item_views_at);
+    float2 *rays = reinterpret_cast<float2 *>(base + rays_at);
+    P->axes = reinterpret_cast<float *>(base + axes_at);
+    P->mask_dev = masked ? reinterpret_cast<uint8_t *>(base + mask_at) : nullptr;
+    P->reps = reinterpret_cast<int4 *>(base + reps_at);
+    P->item_rows = reinterpret_cast<int4 *>(base + rows_at);
+    P->zeros = reinterpret_cast<float *>(base + zeros_at);
+    P->views = views;
+    P->item_views = item_views;
+    P->rays = rays;
+    P->img = reinterpret_cast<float *>(base + img_at);
+    A.splits = sf_default_splits(G, A.nrep, A.fslots, uses != SF_FORWARD);
     // back: about four CTAs of 256 pixels per SM, at least 8 views each
     const long long tiles = (long long)((A.sym.hx + kBackTx - 1) / kBackTx) * ((A.sym.hy + kBackTy - 1) / kBackTy);
     A.gsplit = (int)std::max<long long>(1, std::min<long long>({8, G.na / 8, (4LL * std::max(1, num_sms()) + tiles / 2) / tiles}));
-    SGB_TRY(P->views.reserve(sizeof(SfView) * G.na));
-    SGB_TRY(P->rays.reserve(sizeof(float2) * (size_t)G.na * (G.nb + 1)));
-    sf_setup_views<<<(G.na + 127) / 128, 128, 0, st>>>(G, P->betas.as<double>(), P->views.as<SfView>());
+    const int nview = fwd ? G.na : 0, nset = std::max(nview, (int)items.size());
+    sf_setup_views<<<(nset + 127) / 128, 128, 0, st>>>(G, betas_dev, nview, views, (int)items.size(),
+                                                      reinterpret_cast<int2 *>(base + maps_at), item_views);
     SGB_TRY(after_launch("sf_setup_views"));
-    sf_item_views<<<(A.nitem + 127) / 128, 128, 0, st>>>(items_dev.as<SfItem>(), A.nitem, P->views.as<SfView>(),
-                                                        P->item_views.as<SfView>(), P->item_rows.as<int4>());
-    SGB_TRY(after_launch("sf_item_views"));
-    const long long nr = (long long)G.na * (G.nb + 1);
-    sf_setup_rays<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(G, P->betas.as<double>(), P->views.as<SfView>(),
-                                                                   P->rays.as<float2>());
-    SGB_TRY(after_launch("sf_setup_rays"));
+    if (fwd) {
+        sf_setup_rays<<<(unsigned)((nray + 255) / 256), 256, 0, st>>>(G, betas_dev, views, rays);
+        SGB_TRY(after_launch("sf_setup_rays"));
+    }
     SGB_CUDA(cudaStreamSynchronize(st));
+    out = std::move(P);
+    return SGB_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int sgb_sf_plan_create(const sgb_sino_geom *rg, const sgb_image_geom *ig, sgb_sf_plan **out) {
+    SGB_REQUIRE(out, "sf_plan_create: null argument");
+    *out = nullptr;
+    std::unique_ptr<sgb_sf_plan> P;
+    SGB_TRY(sf_plan(rg, ig, SF_FORWARD | SF_BACK, P));
     *out = P.release();
     return SGB_OK;
 }
@@ -1041,23 +1080,21 @@ int sgb_sf_plan_destroy(sgb_sf_plan *P) {
     return SGB_OK;
 }
 
-// One-shot calls: a plan for the call; they always wait for `stream` before returning.
+// One-shot calls: a plan of one direction for the call; they always wait for `stream` before returning.
 int sgb_sf_project(const sgb_sino_geom *rg, const sgb_image_geom *ig, const float *image, float *sino, int flags,
                    void *stream) {
     SGB_REQUIRE(image && sino, "sf_project: null argument");
-    sgb_sf_plan *P = nullptr;
-    SGB_TRY(sgb_sf_plan_create(rg, ig, &P));
-    std::unique_ptr<sgb_sf_plan> hold(P);
-    return sf_run(P, true, image, sino, flags & ~SGB_ASYNC, static_cast<cudaStream_t>(stream));
+    std::unique_ptr<sgb_sf_plan> P;
+    SGB_TRY(sf_plan(rg, ig, SF_FORWARD, P));
+    return sf_run(P.get(), true, image, sino, flags & ~SGB_ASYNC, static_cast<cudaStream_t>(stream));
 }
 
 int sgb_sf_backproject(const sgb_sino_geom *rg, const sgb_image_geom *ig, const float *sino, float *image, int flags,
                        void *stream) {
     SGB_REQUIRE(image && sino, "sf_backproject: null argument");
-    sgb_sf_plan *P = nullptr;
-    SGB_TRY(sgb_sf_plan_create(rg, ig, &P));
-    std::unique_ptr<sgb_sf_plan> hold(P);
-    return sf_run(P, false, sino, image, flags & ~SGB_ASYNC, static_cast<cudaStream_t>(stream));
+    std::unique_ptr<sgb_sf_plan> P;
+    SGB_TRY(sf_plan(rg, ig, SF_BACK, P));
+    return sf_run(P.get(), false, sino, image, flags & ~SGB_ASYNC, static_cast<cudaStream_t>(stream));
 }
 
 // _tau(rg, x, y), src/geom/tau.jl:7-60 (host, FP64): tau[i + n*v] = projected s/ds of point i in view v.
