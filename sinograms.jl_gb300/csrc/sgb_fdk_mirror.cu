@@ -188,6 +188,17 @@ int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, double l
         T.kz = half ? 32 / ns : 64 / ns;
         T.split = 1;
         const int ntz = floor_div_up(T.nzd, T.kz);
+        const long long ctas = (long long)tx * ty * ntz;
+        auto fits_grid = [&](int g) { return A.nv >= 8 * g && ctas * g <= (1 << 30) && ntz * g <= 65535; };
+        const double edge = edge_share(A, M.iz0, T.kz, !A.quad);
+        // Whatever the boxes are, a launch is predicted to take longer than without any: the pre-pass, some 12 us,
+        // is spared where none can be the fastest (16 x 16 x 4 voxels, 30 views: a plan 380 and 330 us).
+        A.box_bytes = 0;
+        const double least = cta_view(c, A, T.kz, ns, M.nvs, M.zm, edge);
+        double bound = limit_us;
+        for (int g = 1; g <= 8 && fits_grid(g); g *= 2)
+            for (int per = 1; per <= 2; per++) bound = std::min(bound, launch_us(c, least, A.nv, g, ctas, per));
+        if (bound >= best_us) continue;
         SGB_CUDA(cudaMemsetAsync(ext_dev, 0, 2 * sizeof(int), st));
         const long long n = (long long)tx * ty * ntz * T.nviews;
         const unsigned blocks = (unsigned)((n + 255) / 256);
@@ -203,10 +214,8 @@ int fdk_mirror_prepare(FdkMirrorArgs &M, int *ext_dev, cudaStream_t st, double l
         A.box_bytes = (int)(((size_t)A.W * A.H * 8 + 127) / 128 * 128);
         A.nstage = fdk_mirror_smem(T, 4) <= 112 * 1024 ? 4 : 3;
         if (fdk_mirror_smem(T, A.nstage) > 226 * 1024) continue;
-        const double view = cta_view(c, A, T.kz, ns, M.nvs, M.zm, edge_share(A, M.iz0, T.kz, !A.quad));
-        const long long ctas = (long long)tx * ty * ntz;
-        for (int g = 1; g <= 8; g *= 2) {
-            if (A.nv < 8 * g || ctas * g > (1 << 30) || ntz * g > 65535) break;
+        const double view = cta_view(c, A, T.kz, ns, M.nvs, M.zm, edge);
+        for (int g = 1; g <= 8 && fits_grid(g); g *= 2) {
             T.split = g;
             const size_t smem = fdk_mirror_smem(T, A.nstage);
             if (smem > 226 * 1024) break;
